@@ -10,7 +10,7 @@
 //   4. binary radix tree (Karras 2012): internal node i's range and split from common prefixes of the sorted codes
 //   5. boxes, triangle counts and SAH costs bottom-up (each leaf walks towards the root, the second arrival at a node
 //      refits it from its children), then ten such passes that also restructure each node's treelet of up to 7
-//      leaves to its least-SAH topology (Karras & Aila 2013)
+//      leaves to its least-SAH topology (Karras & Aila 2013), a warp per treelet
 //   6. SAH-optimal collapse to 8-wide nodes (Ylitie, Karras & Laine 2017): a bottom-up dynamic program gives each
 //      binary node the least SAH cost of its subtree as at most i = 1..8 children of a wide node, and whether one slot
 //      holds it as a leaf (at most 3 triangles) or as a wide node of its own; level by level, each wide node's children
@@ -176,85 +176,181 @@ __device__ __forceinline__ void refit(const Tree2& T, int x) {
   __stcg(&T.cost[x], n <= kLeafMax ? kCt * A * float(n) : kCi * A + ca + cb);
 }
 
-// Treelet restructuring (Karras & Aila 2013): the treelet of node x has up to 7 leaves (grown by opening the
-// largest-area internal leaf); a dynamic program over the subsets of its leaves finds the binary topology of least SAH
-// cost, and the treelet's internal nodes are rewired to it when that is cheaper. Subsets of at most 3 triangles cost
-// as the one 8-wide leaf they become.
-__device__ void optimize_treelet(const Tree2& T, int x) {
-  int leaf[7], inner[6];
-  int m = 0, ni = 0;
-  inner[ni++] = x;
-  leaf[m++] = __ldcg(&T.left[x]);
-  leaf[m++] = __ldcg(&T.right[x]);
-  while (m < 7) {
-    int best = -1;
-    float bestA = -1.f;
-    for (int k = 0; k < m; ++k) {
-      const int c = leaf[k];
-      if (c < 0 || __ldcg(&T.count[c]) <= kLeafMax) continue;
-      const float A = box_area(__ldcg(&T.nlo[c]), __ldcg(&T.nhi[c]));
-      if (A > bestA) { bestA = A; best = k; }
+// Treelet restructuring (Karras & Aila 2013), a warp per treelet: the treelet of node x has up to 7 leaves (grown by
+// opening the largest-area internal leaf); a dynamic program over the subsets of its leaves finds the binary topology of
+// least SAH cost, and the treelet's internal nodes are rewired to it when that is cheaper. Subsets of at most 3
+// triangles cost as the one 8-wide leaf they become.
+// The pass is bound by latency and issue: some 20 dependent reads and 600 instructions a treelet, a treelet for every
+// node of more than 3 triangles. One thread per treelet, its 127 costs in local memory, kept a warp's lanes on treelets
+// of different shapes for 966 sums each (ten passes over 2 M triangles: 182 ms, this form 17.4 ms);
+// here the lanes share each step: a lane holds a leaf while the treelet grows, four subsets' boxes, one subset's
+// partitions (of the 6- and 7-leaf subsets a part of them), and one node of the new topology.
+constexpr int kTreeletWarps = 4;   // warps a block
+struct Treelet {                   // a warp's shared memory
+  float box[6][8];                 // lo x y z, hi x y z of the leaves (7: none)
+  uint32_t cnt[8];
+  float cost[128];                 // of each subset; before its turn, the part of it that does not depend on the split
+  uint8_t part[128];               // its best split's half
+  uint8_t one[128];                // at most kLeafMax triangles: its cost is that of a leaf
+  uint32_t set[6];                 // the new topology's nodes as subsets, from the root down
+  int node[6], child[6][2];
+};
+// the subsets of 7 leaves by size, and where each size begins
+__constant__ uint8_t kSubset[128] = {
+    0,   1,   2,   4,   8,   16,  32,  64,  3,   5,   6,   9,   10,  12,  17,  18,  20,  24,  33,  34,  36,  40,  48,  65,  66,  68,
+    72,  80,  96,  7,   11,  13,  14,  19,  21,  22,  25,  26,  28,  35,  37,  38,  41,  42,  44,  49,  50,  52,  56,  67,  69,  70,
+    73,  74,  76,  81,  82,  84,  88,  97,  98,  100, 104, 112, 15,  23,  27,  29,  30,  39,  43,  45,  46,  51,  53,  54,  57,  58,
+    60,  71,  75,  77,  78,  83,  85,  86,  89,  90,  92,  99,  101, 102, 105, 106, 108, 113, 114, 116, 120, 31,  47,  55,  59,  61,
+    62,  79,  87,  91,  93,  94,  103, 107, 109, 110, 115, 117, 118, 121, 122, 124, 63,  95,  111, 119, 123, 125, 126, 127};
+__constant__ int kSizeAt[9] = {0, 1, 8, 29, 64, 99, 120, 127, 128};
+
+// the least cost of a split of S and its half that holds S's lowest leaf; `share` lanes (a power of two) work on S, and
+// lane `part` of them takes the halves whose choice of the next lowest leaves is `part`
+__device__ __forceinline__ void best_split(const Treelet& t, uint32_t S, uint32_t part, uint32_t share, float& best, uint32_t& half) {
+  uint32_t fix = S & (0u - S), free = S ^ fix;
+  for (; share > 1; share >>= 1, part >>= 1) {
+    const uint32_t bit = free & (0u - free);
+    if (part & 1u) fix |= bit;
+    free ^= bit;
+  }
+  uint32_t sub = 0;
+  do {   // every subset of the leaves left free
+    const uint32_t P = fix | sub;
+    if (P != S) {
+      const float c = t.cost[P] + t.cost[S ^ P];
+      if (c < best) { best = c; half = P; }
     }
-    if (best < 0) break;
-    const int c = leaf[best];
-    inner[ni++] = c;
-    leaf[best] = __ldcg(&T.left[c]);
-    leaf[m++] = __ldcg(&T.right[c]);
-  }
-  if (m < 4) return;
-  float4 llo[7], lhi[7];
-  uint32_t lcnt[7];
-  float lcost[7];
-  for (int k = 0; k < m; ++k) child_info(T, leaf[k], llo[k], lhi[k], lcnt[k], lcost[k]);
-  float cst[128];
-  uint8_t part[128];
-  const uint32_t full = (1u << m) - 1u;
-  for (uint32_t S = 1; S <= full; ++S) {   // a proper subset precedes its superset
-    float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f), hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
-    uint32_t n = 0;
-    for (int k = 0; k < m; ++k)
-      if (S >> k & 1u) {
-        lo = make_float4(fminf(lo.x, llo[k].x), fminf(lo.y, llo[k].y), fminf(lo.z, llo[k].z), 0.f);
-        hi = make_float4(fmaxf(hi.x, lhi[k].x), fmaxf(hi.y, lhi[k].y), fmaxf(hi.z, lhi[k].z), 0.f);
-        n += lcnt[k];
-      }
-    const uint32_t low = S & (0u - S);
-    if (S == low) { cst[S] = lcost[__ffs(S) - 1]; part[S] = 0; continue; }
-    float best = INFINITY;
-    uint32_t bp = low;
-    for (uint32_t P = (S - 1) & S; P; P = (P - 1) & S)
-      if (P & low) { const float c = cst[P] + cst[S ^ P]; if (c < best) { best = c; bp = P; } }
-    const float A = box_area(lo, hi);
-    cst[S] = n <= kLeafMax ? kCt * A * float(n) : kCi * A + best;
-    part[S] = uint8_t(bp);
-  }
-  if (!(cst[full] < __ldcg(&T.cost[x]) * 0.9999f)) return;   // keep the tree unless the treelet improves
-  // rewire top-down (x stays the root), then refit bottom-up in reverse order of assignment
-  uint32_t setOf[6];
-  int nodeOf[6], order[6];
-  int sp = 0, next = 1, done = 0;
-  setOf[0] = full; nodeOf[0] = x; sp = 1;
-  while (sp) {
-    --sp;
-    const uint32_t S = setOf[sp];
-    const int node = nodeOf[sp];
-    order[done++] = node;
-    const uint32_t P[2] = {part[S], S ^ part[S]};
-    int id[2];
-    for (int h = 0; h < 2; ++h) {
-      if (__popc(P[h]) == 1) id[h] = leaf[__ffs(P[h]) - 1];
-      else { id[h] = inner[next++]; setOf[sp] = P[h]; nodeOf[sp] = id[h]; ++sp; }
-      if (id[h] >= 0) __stcg(&T.parent[id[h]], node); else __stcg(&T.leafParent[~id[h]], node);
-    }
-    __stcg(&T.left[node], id[0]);
-    __stcg(&T.right[node], id[1]);
-  }
-  for (int k = done - 1; k >= 0; --k) refit(T, order[k]);
+    sub = (sub - free) & free;
+  } while (sub);
 }
 
-// bottom-up pass: the second thread to arrive at a node refits it from its children and, when asked, restructures
-// its treelet (every node below is final by then); the first one stops: no thread waits
-__global__ void k_bottom_up(Tree2 T, int n, uint32_t* arrivals, int optimize) {
+__device__ void optimize_treelet(const Tree2& T, int x, Treelet& t, uint32_t lane) {
+  // lane l < m holds leaf l with what opening it needs
+  int leaf = -1, l = 0, r = 0, inner = lane == 0 ? x : -1;
+  float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f), hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+  uint32_t cnt = 0;
+  float cst = 0.f, area = -1.f;
+  const auto hold = [&](int c) {
+    leaf = c;
+    child_info(T, c, lo, hi, cnt, cst);
+    area = -1.f;
+    if (c >= 0 && cnt > kLeafMax) { l = __ldcg(&T.left[c]); r = __ldcg(&T.right[c]); area = box_area(lo, hi); }
+  };
+  if (lane < 2) hold(__ldcg(lane == 0 ? &T.left[x] : &T.right[x]));
+  int m = 2, ni = 1;
+  while (m < 7) {
+    // areas are at least 0 where a leaf can be opened: their bits order as they do, and 0 stands for none
+    const uint32_t key = area >= 0.f ? __float_as_uint(area) + 1u : 0u, top = __reduce_max_sync(~0u, key);
+    if (!top) break;
+    const uint32_t from = __ffs(__ballot_sync(~0u, key == top)) - 1;
+    const int cl = __shfl_sync(~0u, l, from), cr = __shfl_sync(~0u, r, from), c = __shfl_sync(~0u, leaf, from);
+    if (int(lane) == ni) inner = c;
+    if (lane == from || int(lane) == m) hold(lane == from ? cl : cr);
+    ++m;
+    ++ni;
+  }
+  if (m < 4) return;
+  if (lane < 8) {
+    t.box[0][lane] = lo.x; t.box[1][lane] = lo.y; t.box[2][lane] = lo.z;
+    t.box[3][lane] = hi.x; t.box[4][lane] = hi.y; t.box[5][lane] = hi.z;
+    t.cnt[lane] = cnt;
+  }
+  __syncwarp();
+  const uint32_t full = (1u << m) - 1u;
+  {   // the subsets lane + 32 j: leaves 0..4 by the lane's bits, 5 and 6 by j's
+    float b[6];
+    uint32_t n = 0;
+    for (int a = 0; a < 3; ++a) { b[a] = INFINITY; b[3 + a] = -INFINITY; }
+    const auto join = [&](float* q, uint32_t& k, int f) {
+      for (int a = 0; a < 3; ++a) { q[a] = fminf(q[a], t.box[a][f]); q[3 + a] = fmaxf(q[3 + a], t.box[3 + a][f]); }
+      k += t.cnt[f];
+    };
+    for (int f = 0; f < 5; ++f)
+      if (lane >> f & 1u) join(b, n, f);
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+      const uint32_t S = lane + 32 * j;
+      float q[6];
+      uint32_t k = n;
+      for (int a = 0; a < 6; ++a) q[a] = b[a];
+      if (j & 1u) join(q, k, 5);
+      if (j & 2u) join(q, k, 6);
+      const float A = box_area(make_float4(q[0], q[1], q[2], 0.f), make_float4(q[3], q[4], q[5], 0.f));
+      t.one[S] = k <= kLeafMax ? 1 : 0;
+      t.cost[S] = k <= kLeafMax ? kCt * A * float(k) : kCi * A;
+    }
+  }
+  __syncwarp();
+  if (int(lane) < m) t.cost[1u << lane] = cst;
+  __syncwarp();
+  for (int size = 2; size <= m; ++size) {
+    const int at = kSizeAt[size], n = kSizeAt[size + 1] - at;
+    const int share = size == 7 ? 32 : size == 6 ? 4 : 1;   // lanes a subset
+    for (int k0 = 0; k0 < n * share; k0 += 32) {
+      const int k = (k0 + int(lane)) / share;
+      const uint32_t S = k < n ? kSubset[at + k] : 0u;
+      const bool use = S && !(S & ~full);
+      float best = INFINITY;
+      uint32_t half = S & (0u - S);
+      if (use) best_split(t, S, lane & uint32_t(share - 1), uint32_t(share), best, half);
+      for (int o = share / 2; o; o >>= 1) {
+        const float ob = __shfl_xor_sync(~0u, best, o);
+        const uint32_t oh = __shfl_xor_sync(~0u, half, o);
+        if (ob < best || (ob == best && oh < half)) { best = ob; half = oh; }
+      }
+      if (use && (lane & uint32_t(share - 1)) == 0) {
+        if (!t.one[S]) t.cost[S] += best;
+        t.part[S] = uint8_t(half);
+      }
+    }
+    __syncwarp();
+  }
+  if (!(t.cost[full] < __ldcg(&T.cost[x]) * 0.9999f)) return;   // keep the tree unless the treelet improves
+  // the new topology, top-down (x stays the root); the i-th node taken is the treelet's i-th internal node
+  if (int(lane) < ni) t.node[lane] = inner;
+  __syncwarp();
+  if (lane == 0) {
+    int made = 1;
+    t.set[0] = full;
+    for (int i = 0; i < made; ++i) {
+      const uint32_t S = t.set[i], P = t.part[S], half[2] = {P, S ^ P};
+      for (int h = 0; h < 2; ++h) {
+        if (__popc(half[h]) == 1) t.child[i][h] = -int(__ffs(half[h]));   // leaf k as -(k + 1)
+        else { t.child[i][h] = made; t.set[made++] = half[h]; }
+      }
+    }
+  }
+  __syncwarp();
+  if (int(lane) < ni) {   // a lane per node: its children, its box from the leaves', its count and cost
+    const int node = t.node[lane];
+    const uint32_t S = t.set[lane];
+    float4 a = make_float4(INFINITY, INFINITY, INFINITY, 0.f), b = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+    uint32_t n = 0;
+    for (int f = 0; f < m; ++f)
+      if (S >> f & 1u) {
+        a = make_float4(fminf(a.x, t.box[0][f]), fminf(a.y, t.box[1][f]), fminf(a.z, t.box[2][f]), 0.f);
+        b = make_float4(fmaxf(b.x, t.box[3][f]), fmaxf(b.y, t.box[4][f]), fmaxf(b.z, t.box[5][f]), 0.f);
+        n += t.cnt[f];
+      }
+    __stcg(&T.nlo[node], a);
+    __stcg(&T.nhi[node], b);
+    __stcg(&T.count[node], n);
+    __stcg(&T.cost[node], t.cost[S]);
+  }
+  for (int i = 0; i < ni; ++i)
+    for (int h = 0; h < 2; ++h) {
+      const int c = t.child[i][h];
+      const int id = c >= 0 ? t.node[c] : __shfl_sync(~0u, leaf, -c - 1);   // c is the same for every lane
+      if (lane == 0) {
+        __stcg(h == 0 ? &T.left[t.node[i]] : &T.right[t.node[i]], id);
+        __stcg(id >= 0 ? &T.parent[id] : &T.leafParent[~id], t.node[i]);
+      }
+    }
+}
+
+// bottom-up pass: the second thread to arrive at a node refits it from its children (every node below is final by
+// then); the first one stops: no thread waits
+__global__ void k_bottom_up(Tree2 T, int n, uint32_t* arrivals) {
   const int p = int(blockIdx.x * blockDim.x + threadIdx.x);
   if (p >= n) return;
   int node = __ldcg(&T.leafParent[p]);
@@ -263,9 +359,39 @@ __global__ void k_bottom_up(Tree2 T, int n, uint32_t* arrivals, int optimize) {
     if (atomicAdd(&arrivals[node], 1u) == 0) return;
     __threadfence();
     refit(T, node);
-    if (optimize && __ldcg(&T.count[node]) > kLeafMax) optimize_treelet(T, node);
     __threadfence();
     node = __ldcg(&T.parent[node]);
+  }
+}
+// the same with each node's treelet restructured once it is refit: a warp's threads walk up together, and the warp
+// restructures the treelets of those that arrived second one after the other
+__global__ void __launch_bounds__(32 * kTreeletWarps) k_treelets(Tree2 T, int n, uint32_t* arrivals) {
+  __shared__ Treelet shared[kTreeletWarps];
+  Treelet& t = shared[threadIdx.x / 32];
+  const uint32_t lane = threadIdx.x & 31;
+  const int p = int(blockIdx.x * blockDim.x + threadIdx.x);
+  int node = p < n ? __ldcg(&T.leafParent[p]) : -1;
+  while (__any_sync(~0u, node >= 0)) {
+    bool work = false;
+    if (node >= 0) {
+      __threadfence();
+      if (atomicAdd(&arrivals[node], 1u) == 0) node = -1;
+      else {
+        __threadfence();
+        refit(T, node);
+        work = __ldcg(&T.count[node]) > kLeafMax;
+      }
+    }
+    __threadfence();
+    uint32_t todo = __ballot_sync(~0u, work);
+    while (todo) {
+      const int from = __ffs(todo) - 1;
+      todo &= todo - 1;
+      optimize_treelet(T, __shfl_sync(~0u, node, from), t, lane);
+      __threadfence();
+      __syncwarp();
+    }
+    if (node >= 0) node = __ldcg(&T.parent[node]);
   }
 }
 
@@ -514,7 +640,8 @@ std::string build_bvh8_gpu(const float* v, size_t nv, const uint32_t* tri, size_
     // 5. boxes, counts, costs; then passes of treelet restructuring
     for (int pass = 0; pass <= kTreeletPasses; ++pass) {
       KGB_TRY(cudaMemsetAsync(arr.p, 0, ni * 4, st));
-      k_bottom_up<<<unsigned(tiles), 256, 0, st>>>(T2, n, arr.as<uint32_t>(), pass > 0 ? 1 : 0);
+      if (!pass) k_bottom_up<<<unsigned(tiles), 256, 0, st>>>(T2, n, arr.as<uint32_t>());
+      else k_treelets<<<unsigned((nt + 32 * kTreeletWarps - 1) / (32 * kTreeletWarps)), 32 * kTreeletWarps, 0, st>>>(T2, n, arr.as<uint32_t>());
     }
   }
   // 6a. the collapse's program, bottom-up over the final tree
