@@ -3,9 +3,9 @@
 // inner child until it has 8) with float child boxes, stored as the 208-byte node / 48-byte triangle records rt.cuh
 // reads.
 //
-// Conservative by construction: every triangle box is expanded by 2^-16 x the scene's largest coordinate (256 ulps at
-// that magnitude) before anything is built, so a box test never drops a triangle the watertight test would report;
-// the traversal then equals the brute-force hit set on any input.
+// Conservative by construction: every triangle box is expanded by prim_eps (engine.h; the bound is at kWiden in rt.cuh)
+// before anything is built, so a box test never drops a triangle the watertight test would report; the traversal then
+// equals the brute-force hit set on any input.
 #include "engine.h"
 
 #include <algorithm>
@@ -95,13 +95,19 @@ void build_bvh8(const float* v, size_t nv, const uint32_t* tri, size_t nt, const
   Builder B;
   float M = 1.f;
   for (size_t k = 0; k < 3 * nv; ++k) M = std::max(M, std::fabs(v[k]));
-  const float eps = M * (1.f / 65536.f);
   B.tb.resize(nt); B.cen.resize(3 * nt); B.idx.resize(nt);
   for (size_t k = 0; k < nt; ++k) {
     B.idx[k] = uint32_t(k);
+    const float* p[3] = {v + 3 * size_t(tri[3 * k]), v + 3 * size_t(tri[3 * k + 1]), v + 3 * size_t(tri[3 * k + 2])};
+    float L = 0.f, e1[3], e2[3];
     for (int a = 0; a < 3; ++a) {
-      const float x0 = v[3 * tri[3 * k] + a], x1 = v[3 * tri[3 * k + 1] + a], x2 = v[3 * tri[3 * k + 2] + a];
-      const float lo = std::min({x0, x1, x2}), hi = std::max({x0, x1, x2});
+      e1[a] = p[1][a] - p[0][a]; e2[a] = p[2][a] - p[0][a];
+      L = std::max({L, std::fabs(e1[a]), std::fabs(e2[a]), std::fabs(p[2][a] - p[1][a])});
+    }
+    const float nx = e1[1] * e2[2] - e1[2] * e2[1], ny = e1[2] * e2[0] - e1[0] * e2[2], nz = e1[0] * e2[1] - e1[1] * e2[0];
+    const float eps = prim_eps(L, std::sqrt(nx * nx + ny * ny + nz * nz), M);
+    for (int a = 0; a < 3; ++a) {
+      const float lo = std::min({p[0][a], p[1][a], p[2][a]}), hi = std::max({p[0][a], p[1][a], p[2][a]});
       B.tb[k].lo[a] = lo - eps; B.tb[k].hi[a] = hi + eps;
       B.cen[3 * k + a] = 0.5f * lo + 0.5f * hi;
     }

@@ -4,8 +4,8 @@
 // 8-wide nodes with float child boxes and the 48-byte triangle records that rt.cuh reads, the same layout as the host
 // builder (bvh_build.cpp) makes.
 //
-//   1. |coordinates| maximum -> eps = max(1, M) / 65536 (the host builder's expansion)
-//   2. per triangle: box (expanded by eps), centroid; centroid bounds
+//   1. M, the largest |coordinate|, at least 1
+//   2. per triangle: box (expanded by prim_eps, as the host builder), centroid; centroid bounds
 //   3. 63-bit Morton codes of the centroids, radix-sorted with the triangle index (stable: ties keep index order)
 //   4. binary radix tree (Karras 2012): internal node i's range and split from common prefixes of the sorted codes
 //   5. boxes, triangle counts and SAH costs bottom-up (each leaf walks towards the root, the second arrival at a node
@@ -51,13 +51,19 @@ __global__ void k_maxabs(const float* v, size_t n, uint32_t* out) {
 }
 
 // triangle boxes (expanded), centroids (of the unexpanded box, as the host), centroid bounds (ordered uints)
-__global__ void k_prims(const float* v, const uint32_t* tri, uint32_t nt, float eps, float4* lo, float4* hi, float4* cen, uint32_t* cb) {
+__global__ void k_prims(const float* v, const uint32_t* tri, uint32_t nt, float M, float4* lo, float4* hi, float4* cen, uint32_t* cb) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t cmin[3] = {~0u, ~0u, ~0u}, cmax[3] = {0u, 0u, 0u};
   if (t < nt) {
     float l[3], h[3], c[3];
+    const float *p0 = v + 3 * size_t(tri[3 * size_t(t)]), *p1 = v + 3 * size_t(tri[3 * size_t(t) + 1]), *p2 = v + 3 * size_t(tri[3 * size_t(t) + 2]);
+    const float ax = p1[0] - p0[0], ay = p1[1] - p0[1], az = p1[2] - p0[2], bx = p2[0] - p0[0], by = p2[1] - p0[1], bz = p2[2] - p0[2];
+    const float L = fmaxf(fmaxf(fmaxf(fabsf(ax), fabsf(ay)), fmaxf(fabsf(az), fabsf(bx))),
+                          fmaxf(fmaxf(fabsf(by), fabsf(bz)), fmaxf(fabsf(p2[0] - p1[0]), fmaxf(fabsf(p2[1] - p1[1]), fabsf(p2[2] - p1[2])))));
+    const float nx = ay * bz - az * by, ny = az * bx - ax * bz, nz = ax * by - ay * bx;
+    const float eps = prim_eps(L, sqrtf(nx * nx + ny * ny + nz * nz), M);
     for (int a = 0; a < 3; ++a) {
-      const float x0 = v[3 * tri[3 * t] + a], x1 = v[3 * tri[3 * t + 1] + a], x2 = v[3 * tri[3 * t + 2] + a];
+      const float x0 = p0[a], x1 = p1[a], x2 = p2[a];
       const float mn = fminf(x0, fminf(x1, x2)), mx = fmaxf(x0, fmaxf(x1, x2));
       l[a] = __fsub_rn(mn, eps); h[a] = __fadd_rn(mx, eps);
       c[a] = __fadd_rn(__fmul_rn(0.5f, mn), __fmul_rn(0.5f, mx));
@@ -604,13 +610,12 @@ std::string build_bvh8_gpu(const float* v, size_t nv, const uint32_t* tri, size_
   float M;
   std::memcpy(&M, &mbits, 4);
   M = std::max(1.f, M);
-  const float eps = M * (1.f / 65536.f);
   // 2. boxes, centroids, centroid bounds
   KGB_TRY(cudaMalloc(&plo.p, nt * 16)); KGB_TRY(cudaMalloc(&phi.p, nt * 16)); KGB_TRY(cudaMalloc(&cen.p, nt * 16));
   KGB_TRY(cudaMalloc(&cb.p, 24));
   const uint32_t cbInit[6] = {~0u, ~0u, ~0u, 0u, 0u, 0u};
   KGB_TRY(cudaMemcpyAsync(cb.p, cbInit, 24, cudaMemcpyHostToDevice, st));
-  k_prims<<<unsigned(tiles), 256, 0, st>>>(dv.as<float>(), dtri.as<uint32_t>(), uint32_t(nt), eps, plo.as<float4>(), phi.as<float4>(), cen.as<float4>(),
+  k_prims<<<unsigned(tiles), 256, 0, st>>>(dv.as<float>(), dtri.as<uint32_t>(), uint32_t(nt), M, plo.as<float4>(), phi.as<float4>(), cen.as<float4>(),
                                            cb.as<uint32_t>());
   // 3. Morton codes, sorted
   KGB_TRY(cudaMalloc(&keys.p, nt * 8)); KGB_TRY(cudaMalloc(&keys2.p, nt * 8));

@@ -4,8 +4,7 @@
 // Numerics contract: the code deciding a result (hit or miss, t, own plane, transmittance byte, direction cell, sky
 // bin) is a fixed sequence of IEEE-754 float operations: this header is compiled with -fmad=false and divisions /
 // square roots are the correctly rounded ones, so the results equal a host restatement compiled without contraction
-// bit for bit. Box tests only filter: they are conservative (boxes expanded at build, see bvh_build.cpp) and may use
-// fused operations.
+// bit for bit. Box tests only filter: they are conservative (see kWiden) and may use fused operations.
 #pragma once
 #include <cfloat>
 #include <cstdint>
@@ -283,15 +282,32 @@ __device__ __forceinline__ unsigned long long pku(uint32_t a, uint32_t b) {
 #endif
 }
 
+// What the box test owes a hit that the triangle test computes, with u = 2^-24 (a float's half ulp), t the hit's
+// distance, L the triangle's extent, M the scene's largest coordinate:
+//  - the watertight test signs its edge functions exactly for vertices slightly off where they are relative to the ray:
+//    subtracting the origin, shearing and rounding the result move them by at most 4 u t |d_a| + 6 u L along axis a
+//    (Sx times the depth is t |d_a| up to L, and so is the vertex's offset). So the ray passes within that of the triangle,
+//    and 4 u t |d_a| is 4 u of the axis's slab distance;
+//  - a slab distance fma(plane, 1 / d, -o / d) is off by 3 u of itself and, for a coordinate |o_a| up to 6 M, by 7 u M in
+//    distance (the products' rounding and the planes'); past 6 M that too is a small part of the slab distance;
+//  - the computed t is off by about 8 u of itself and by a few u L, times L^2 / area for a sliver.
+// The exit distance is widened by kWiden, 1 + 32 u, which covers the parts relative to t on both sides of the interval;
+// the triangles' boxes are expanded by prim_eps (8 u M and 32 u L L^2 / area), which covers the others.
+// Every box used to be expanded by 256 u M: 6 mm on a 400 m block, more than the 0.1 to 4 mm by which offset_ray lifts
+// a sensor off its face, so every ray began inside the boxes of its own wall and walked down to its triangles. With the
+// walls' boxes behind the sensors the urban block's rays visit about 6.9 nodes instead of 8.2 and test 0.9 triangles instead
+// of 1.9 (trace 57.5 to 43.3 ms); rotated walls' boxes hold their sensors either way.
+constexpr float kWiden = 1.0000019073486328125f;   // 1 + 2^-19
+
 // Child boxes of the node at p against the ray in [tmin, tmax] (tmin >= 0): returns the mask of hit children (bit k),
 // their entry distances in tn[8]. Per axis the slab distance of a plane is fma(plane, inv, -o inv); the near planes
 // are the low ones when inv >= 0, else the high ones, and the ray's nearX.. index picks their vector (the far one is
 // the other). Children go in pairs through the packed fma: per pair one fma.f32x2 per plane, per child one 3-input max
-// and one 3-input min. Conservative: the triangle boxes were expanded at build by 2^-16 of the scene's largest
-// coordinate, far beyond the rounding of these distances, and the exit distance is widened by 2^-20 besides. Empty
-// child slots (lo +inf, hi -inf) fail the test; a leaf slot without triangles that passes tests nothing.
-// CLIP: the exit is also clipped at tmax (closest hit, where tmax shrinks to the best hit). Without it boxes beyond
-// tmax pass as well, which is conservative: the triangle test applies tmax (the any-hit walks run to infinity).
+// and one 3-input min. Empty child slots (lo +inf, hi -inf) fail the test; a leaf slot without triangles that passes
+// tests nothing.
+// CLIP: the exit is also clipped at tmax (closest hit: the best hit so far times kWiden, as a box's entry may lie that
+// much past a hit in it). Without it boxes beyond tmax pass as well, which is conservative: the triangle test applies
+// tmax (the any-hit walks run to infinity).
 // 1 + the node's last slot in use, from bit 7 of its first three meta bytes (the word of meta[0..3]).
 __device__ __forceinline__ uint32_t node_slots(uint32_t meta03) {
   return 1u + (((meta03 >> 7) & 1u) | ((meta03 >> 14) & 2u) | ((meta03 >> 21) & 4u));
@@ -305,7 +321,7 @@ template <bool CLIP = true, bool SKIP = false>
 __device__ __forceinline__ uint32_t node_hits(const uint4* p, const Ray& r, float tmin, float tmax, uint32_t slots, float* tn) {
   const unsigned long long IX = pk2(r.inv.x, r.inv.x), IY = pk2(r.inv.y, r.inv.y), IZ = pk2(r.inv.z, r.inv.z);
   const unsigned long long OX = pk2(-r.oinv.x, -r.oinv.x), OY = pk2(-r.oinv.y, -r.oinv.y), OZ = pk2(-r.oinv.z, -r.oinv.z);
-  const unsigned long long WIDEN = pk2(1.00000095367431640625f, 1.00000095367431640625f);
+  const unsigned long long WIDEN = pk2(kWiden, kWiden);
   const uint32_t fX = r.nearX ^ 2u, fY = r.nearY ^ 2u, fZ = r.nearZ ^ 2u;
   uint32_t mask = 0;
 #pragma unroll
@@ -325,8 +341,7 @@ __device__ __forceinline__ uint32_t node_hits(const uint4* p, const Ray& r, floa
       up2(fma2(j ? pku(fy.z, fy.w) : pku(fy.x, fy.y), IY, OY), tfy[0], tfy[1]);
       up2(fma2(j ? pku(nz.z, nz.w) : pku(nz.x, nz.y), IZ, OZ), tnz[0], tnz[1]);
       up2(fma2(j ? pku(fz.z, fz.w) : pku(fz.x, fz.y), IZ, OZ), tfz[0], tfz[1]);
-      // exit widened to tfar (1 + 2^-20): for tfar >= 0 the value fma(|tfar|, 2^-20, tfar), and a negative tfar fails
-      // against tnear >= tmin >= 0 either way
+      // exit widened to tfar kWiden; a negative tfar fails against tnear >= tmin >= 0 either way
       float tf[2];
       up2(mul2(pk2(min3f(tfx[0], tfy[0], tfz[0]), min3f(tfx[1], tfy[1], tfz[1])), WIDEN), tf[0], tf[1]);
 #pragma unroll
@@ -442,7 +457,7 @@ __device__ __forceinline__ bool closest(const Scene& s, const Ray& r, float tmin
   Entry stack[kStack * 4];
   int sp = 0;
   bool any = false;
-  float best = tmax;
+  float best = tmax, lim = tmax * kWiden;   // lim: the boxes' bound on the entry distance
   uint32_t cur = 0, visits = 0;
   const uint32_t cap = visit_cap(s);
   for (;;) {
@@ -450,7 +465,7 @@ __device__ __forceinline__ bool closest(const Scene& s, const Ray& r, float tmin
     const uint4* np = reinterpret_cast<const uint4*>(s.nodes + cur);
     const uint4 hd = __ldg(np);
     float tn[8];
-    const uint32_t hit = node_hits<true, SKIP>(np, r, tmin, best, SKIP ? node_slots(hd.z) : 8u, tn);
+    const uint32_t hit = node_hits<true, SKIP>(np, r, tmin, lim, SKIP ? node_slots(hd.z) : 8u, tn);
     const uint32_t imask = hd.x >> 24, childBase = hd.x & 0xffffffu;
     uint32_t leaves = hit & ~imask;
     while (leaves) {
@@ -469,6 +484,7 @@ __device__ __forceinline__ bool closest(const Scene& s, const Ray& r, float tmin
             out.h = h; out.v0 = v0; out.v1 = v1; out.v2 = v2; out.flags = flags; out.slot = slot;
             any = true;
             best = h.t;
+            lim = best * kWiden;
           }
         }
       }
@@ -480,7 +496,7 @@ __device__ __forceinline__ bool closest(const Scene& s, const Ray& r, float tmin
     while (inner) {
       const int k = __ffs(inner) - 1;
       inner &= inner - 1;
-      if (tn[k] > best) continue;
+      if (tn[k] > lim) continue;
       const Entry x{childBase + __popc(imask & ((1u << k) - 1u)), tn[k]};
       int b = m - 1;
       while (b >= 0 && ch[b].t < x.t) { ch[b + 1] = ch[b]; --b; }
@@ -496,7 +512,7 @@ __device__ __forceinline__ bool closest(const Scene& s, const Ray& r, float tmin
     for (;;) {   // the next pushed node still in front of the best hit
       if (!sp) return any;
       const Entry e = stack[--sp];
-      if (e.t <= best) { cur = e.node; break; }
+      if (e.t <= lim) { cur = e.node; break; }
     }
   }
 }
