@@ -814,10 +814,11 @@ KGB_API int kgb_reduce(kgb_engine* e, size_t nc, const float* W, int useCos, dou
   if (!upload(g.scratch, W, g.nDir * 4, g.st) || !grow(g.out, nc * 8) || !grow(g.w64, g.nDir * 8)) return 0;
   const float* N = static_cast<const float*>(g.N.p) + 3 * g.i0;
   double* w64 = static_cast<double*>(g.w64.p);
+  const bool plain = plain_weights(W, g.nDir);
   if (g.bytes) launch_reduce_bytes(static_cast<const uint8_t*>(g.vis.p), uint32_t(nc), uint32_t(g.nDir), N, static_cast<const float*>(g.D.p),
-                                   static_cast<const float*>(g.scratch.p), useCos, static_cast<double*>(g.out.p), g.st, w64);
+                                   static_cast<const float*>(g.scratch.p), useCos, static_cast<double*>(g.out.p), g.st, w64, plain);
   else launch_reduce_bits(static_cast<const uint32_t*>(g.vis.p), uint32_t(nc), uint32_t(g.nWords), uint32_t(g.nDir), N, static_cast<const float*>(g.D.p),
-                          static_cast<const float*>(g.scratch.p), useCos, static_cast<double*>(g.out.p), g.st, w64);
+                          static_cast<const float*>(g.scratch.p), useCos, static_cast<double*>(g.out.p), g.st, w64, plain);
   CU(cudaGetLastError());
   CU(cudaMemcpyAsync(out, g.out.p, nc * 8, cudaMemcpyDeviceToHost, g.st));
   CU(cudaStreamSynchronize(g.st));
@@ -1212,8 +1213,9 @@ KGB_API int kgb_reduce_dc(kgb_engine* e, size_t nc, const float* W, double* out)
   Engine& g = *E(e);
   if (nc == 0) return 1;
   if (nc != g.dcN) return fail("gpu_reduce_dc: no gpu_bounce rows for this chunk");
-  if (!upload(g.scratch, W, g.nBins * 4, g.st) || !grow(g.out, nc * 8)) return 0;
-  launch_reduce_dc(static_cast<const float*>(g.dc.p), uint32_t(nc), uint32_t(g.nBins), static_cast<const float*>(g.scratch.p), static_cast<double*>(g.out.p), g.st);
+  if (!upload(g.scratch, W, g.nBins * 4, g.st) || !grow(g.out, nc * 8) || !grow(g.w64, g.nBins * 8)) return 0;
+  launch_reduce_dc(static_cast<const float*>(g.dc.p), uint32_t(nc), uint32_t(g.nBins), static_cast<const float*>(g.scratch.p), static_cast<double*>(g.out.p),
+                   g.st, static_cast<double*>(g.w64.p), plain_weights(W, g.nBins));
   CU(cudaGetLastError());
   CU(cudaMemcpyAsync(out, g.out.p, nc * 8, cudaMemcpyDeviceToHost, g.st));
   CU(cudaStreamSynchronize(g.st));

@@ -118,13 +118,19 @@ size_t bounce_state_bytes();   // one queued path
 int bounce_step_blocks_per_sm();
 
 // reductions (reduce.cu)
-// w64: a device array of nDir doubles for the weights (the fast form), or null (the weights staged per block in
-// shared memory: for callers with no room for the array)
+// w64: a device array of nDir doubles for the weights, or null (the weights staged per block in shared memory: for callers
+// with no room for the array). plain (with w64): every weight is zero or a positive normal float, so that the sums can
+// run in integer arithmetic (the same bits).
+inline bool plain_weights(const float* W, size_t n) {
+  bool ok = true;
+  for (size_t k = 0; k < n; ++k) ok &= W[k] == 0.f || (W[k] >= 1.17549435e-38f && W[k] <= 3.40282347e38f);
+  return ok;
+}
 void launch_reduce_bits(const uint32_t* bits, uint32_t nc, uint32_t nWords, uint32_t nDir, const float* N, const float* D, const float* W,
-                        int useCos, double* out, cudaStream_t st, double* w64 = nullptr);
+                        int useCos, double* out, cudaStream_t st, double* w64 = nullptr, bool plain = false);
 void launch_reduce_bytes(const uint8_t* bytes, uint32_t nc, uint32_t nDir, const float* N, const float* D, const float* W, int useCos,
-                         double* out, cudaStream_t st, double* w64 = nullptr);
-void launch_reduce_dc(const float* dc, uint32_t nc, uint32_t nBins, const float* W, double* out, cudaStream_t st);
+                         double* out, cudaStream_t st, double* w64 = nullptr, bool plain = false);
+void launch_reduce_dc(const float* dc, uint32_t nc, uint32_t nBins, const float* W, double* out, cudaStream_t st, double* w64, bool plain);
 struct ViewReduceArgs {
   const uint8_t* cls;
   const float* dist;

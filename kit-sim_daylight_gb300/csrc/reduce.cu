@@ -7,6 +7,7 @@
 // The summation orders are fixed (direction order per thread; lane order + shuffle tree per warp), so a sensor's
 // doubles do not depend on the chunk it is in, and equal the oracle's restatement bit for bit.
 #include "engine.h"
+#include "ordered_sum.cuh"
 #include "rt.cuh"
 
 namespace kgb {
@@ -287,26 +288,193 @@ __global__ void __launch_bounds__(kReduceBlock) k_reduce_bytes_w64(const uint8_t
   out[i] = acc;
 }
 
+// The sums in integer arithmetic (ordered_sum.cuh: the same bits), for weights that are zero or positive normal floats; a
+// direction's weight is (significand, biased exponent). Terms gives what a sensor's term of a direction is made from
+// (raw), read ahead of its use, and its factor; where a factor is not a normal float (a normal of almost no length), the
+// sensor's sum is done again with FP64 fmas.
+__global__ void k_weight_parts(const float* __restrict__ W, uint32_t n, uint2* __restrict__ out) {
+  const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
+  if (d >= n) return;
+  const uint32_t b = __float_as_uint(W[d]);
+  out[d] = (b & 0x7fffffffu) ? make_uint2(os_sig(b), b >> 23) : make_uint2(0u, 1u);
+}
+__device__ __forceinline__ double part_weight(uint2 w) { return w.x ? (double)__uint_as_float((w.y << 23) | (w.x & 0x7fffffu)) : 0.0; }
+
+template <bool COS>
+struct BitsTerms {   // a visibility bit: the cosine, or 1
+  const uint32_t* bits;
+  uint32_t nc;
+  const float *N, *D;
+  using Raw = uint32_t;   // the word that holds the direction's bit
+  __device__ __forceinline__ F3 sensor(uint32_t i) const { return COS ? ld3(N + 3 * size_t(i)) : f3(0.f, 0.f, 0.f); }
+  __device__ __forceinline__ Raw raw(uint32_t d, uint32_t i) const { return __ldg(bits + size_t(d / 32) * nc + i); }
+  __device__ __forceinline__ float factor(Raw m, uint32_t d, float c) const { return (m >> (d & 31u)) & 1u ? c : 0.f; }
+};
+template <bool COS>
+struct BytesTerms {   // a transmittance byte: the cosine or 1 times b / 255
+  const uint8_t* bytes;
+  uint32_t nc;
+  const float *N, *D;
+  using Raw = uint32_t;
+  __device__ __forceinline__ F3 sensor(uint32_t i) const { return COS ? ld3(N + 3 * size_t(i)) : f3(0.f, 0.f, 0.f); }
+  __device__ __forceinline__ Raw raw(uint32_t d, uint32_t i) const { return __ldg(bytes + size_t(d) * nc + i); }
+  __device__ __forceinline__ float factor(Raw b, uint32_t, float c) const { return b ? c * (float(b) / 255.f) : 0.f; }
+};
+struct DcTerms {   // a sky bin's reflected light
+  const float* dc;
+  uint32_t nc;
+  const float* D;   // none
+  using Raw = float;
+  __device__ __forceinline__ F3 sensor(uint32_t) const { return f3(0.f, 0.f, 0.f); }
+  __device__ __forceinline__ Raw raw(uint32_t d, uint32_t i) const { return __ldg(dc + size_t(d) * nc + i); }
+  __device__ __forceinline__ float factor(Raw x, uint32_t, float) const { return x; }
+};
+template <bool COS> __device__ __forceinline__ float cosine(F3 n, F3 d) { return COS ? fmaxf(dotf(n, d), 0.f) : 1.f; }
+
+__device__ __forceinline__ void term(float x, uint2 w, uint64_t& p, int32_t& e, bool& odd) {
+  const uint32_t b = __float_as_uint(x);
+  odd = odd || (x != 0.f && os_odd(b));
+  p = x != 0.f ? uint64_t(os_sig(b)) * w.x : 0ull;
+  e = int32_t((b >> 23) + w.y);
+}
+template <bool COS, class S>
+__device__ __noinline__ double fp64_sum(const S& s, uint32_t n, const uint2* W, uint32_t i) {
+  const F3 v = s.sensor(i);
+  double acc = 0;
+  for (uint32_t d = 0; d < n; ++d) {
+    const float x = s.factor(s.raw(d, i), d, cosine<COS>(v, COS ? ld3(s.D + 3 * d) : F3{}));
+    if (x != 0.f) acc = __fma_rn((double)x, part_weight(W[d]), acc);
+  }
+  return acc;
+}
+
+// A warp for a sensor, a lane per direction. While a sum's exponent stays, every term can be rounded by itself and the
+// rounded terms added in any order: each lane rounds its own, and the warp adds them up. A term halfway between two
+// values goes to the even one, which depends on the parity of the sum before it: the parity of the rounded terms since
+// the last such term (which left an even sum) or since the 32 began. The term that starts the sum, one that lies above
+// the sum's grid and one that takes the sum into the next binade are added alone, between those before and after.
+__device__ __forceinline__ void add_32(OrderedSum& s, uint64_t p, int32_t e, uint32_t lane) {
+  uint32_t todo = __ballot_sync(~0u, p != 0);
+  const auto alone = [&](int from) {
+    const uint64_t q = uint64_t(__shfl_sync(~0u, uint32_t(p), from)) | uint64_t(__shfl_sync(~0u, uint32_t(p >> 32), from)) << 32;
+    os_add(s, q, __shfl_sync(~0u, e, from));
+    todo &= ~1u << from;
+  };
+  while (todo) {
+    if (!s.a) { alone(__ffs(todo) - 1); continue; }
+    const int32_t sh = s.g - e;
+    const uint32_t by = uint32_t(sh) < 63u ? uint32_t(sh) : 63u, below = (1u << lane) - 1u, above = __ballot_sync(~0u, sh < 0) & todo;
+    const uint32_t now = above ? todo & ((above & (0u - above)) - 1u) : todo;   // the terms before the first one above the grid
+    const bool mine = now >> lane & 1u;
+    const uint64_t rem = (p << (63u - by)) << 1, half = 1ull << 63;
+    uint64_t r = mine ? (p >> by) + (rem > half ? 1u : 0u) : 0ull;   // at most 2^48
+    const uint32_t ties = __ballot_sync(~0u, mine && rem == half);
+    if (ties) {
+      const uint32_t odd = __ballot_sync(~0u, uint32_t(r) & 1u), last = ties & below;
+      const uint32_t since = last ? below & (~1u << (31 - __clz(last))) : below;
+      const uint32_t before = (__popc(odd & since) & 1u) ^ (last ? 0u : uint32_t(s.a) & 1u);
+      if (ties >> lane & 1u) r += before ^ (uint32_t(r) & 1u);
+    }
+    const uint64_t a = s.a + __reduce_add_sync(~0u, uint32_t(r) & 0xffffffu) + (uint64_t(__reduce_add_sync(~0u, uint32_t(r >> 24))) << 24);
+    if (!(a >> 53)) {
+      s.a = a;
+      todo &= ~now;
+      if (above) alone(__ffs(above) - 1);
+      continue;
+    }
+    uint64_t upTo = r;   // the sum of the terms up to and with the lane's
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint64_t x = uint64_t(__shfl_up_sync(~0u, uint32_t(upTo), o)) | uint64_t(__shfl_up_sync(~0u, uint32_t(upTo >> 32), o)) << 32;
+      if (lane >= uint32_t(o)) upTo += x;
+    }
+    const int past = __ffs(__ballot_sync(~0u, (s.a + upTo) >> 53)) - 1;
+    const uint64_t less = upTo - r;
+    s.a += uint64_t(__shfl_sync(~0u, uint32_t(less), past)) | uint64_t(__shfl_sync(~0u, uint32_t(less >> 32), past)) << 32;
+    alone(past);   // and the terms before it are done
+  }
+}
+// Four warps a block, and four words of directions read before any is added: a warp alone on its SM quarter is bound by the
+// latency of its reads, many of them by issue, some 150 slots a word.
+constexpr uint32_t kSumWarps = 4;
+constexpr int kAhead = 4;
+template <bool COS, class S>
+__global__ void __launch_bounds__(32 * kSumWarps) k_sum_warp(S t, uint32_t n, const uint2* __restrict__ W, double* __restrict__ out) {
+  const uint32_t i = blockIdx.x * kSumWarps + threadIdx.x / 32, lane = threadIdx.x & 31;
+  if (i >= t.nc) return;   // whole warps
+  const F3 v = t.sensor(i);
+  OrderedSum s;
+  bool odd = false;
+  for (uint32_t d0 = 0; d0 < n; d0 += 32 * kAhead) {
+    typename S::Raw raw[kAhead];
+    F3 dir[kAhead];
+    uint2 w[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const uint32_t d = min(d0 + 32 * k + lane, n - 1);
+      raw[k] = t.raw(d, i);
+      if (COS) dir[k] = ld3(t.D + 3 * d);
+      w[k] = __ldg(W + d);
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const uint32_t d = d0 + 32 * k + lane;
+      uint64_t p;
+      int32_t e;
+      term(d < n ? t.factor(raw[k], d, cosine<COS>(v, dir[k])) : 0.f, w[k], p, e, odd);
+      add_32(s, p, e, lane);
+    }
+  }
+  odd = __any_sync(~0u, odd);
+  if (lane) return;
+  out[i] = odd ? fp64_sum<COS>(t, n, W, i) : __longlong_as_double((long long)os_bits(s));
+}
+
+static uint32_t blocks_of(uint32_t n) { return (n + kReduceBlock - 1) / kReduceBlock; }
+template <bool COS, class S>
+static void launch_sum_warp(const S& t, uint32_t n, const float* W, double* w64, double* out, cudaStream_t st) {
+  uint2* parts = reinterpret_cast<uint2*>(w64);
+  k_weight_parts<<<(n + 255) / 256, 256, 0, st>>>(W, n, parts);
+  k_sum_warp<COS><<<(t.nc + kSumWarps - 1) / kSumWarps, 32 * kSumWarps, 0, st>>>(t, n, parts, out);
+}
+// Which form is faster (152 SMs): the thread form waits some 70 ns a direction for its fma and its reads (bits without
+// the cosine; 110 ns with it, 140 and 180 ns bytes), whatever the sensors, until they fill the SMs; the warp form costs
+// a sensor 7 us / 100,000 for each word of 32 directions and for a hundred words' worth more at the start of its sum,
+// where nearly every term doubles it. Measured, both forms, us a call: 12,345 sensors x 5610 directions 793 / 378
+// (cosine), 485 / 329; 20,000 x 5610 753 / 556, 481 / 481; 40,000 x 5610 776 / 1016, 490 / 880; 12,345 x 2155
+// 289 / 194, 182 / 180; 12,000 x 100 45 / 67; bytes 20,011 x 9066 1772 / 842, 1382 / 712; 32,000 x 2155 477 / 477.
+// Under 256 directions the start of the sum is most of it (16 sensors x 15 directions: 5 us against 14).
+static bool warp_sums(uint32_t nc, uint32_t n, uint32_t rate) { return n >= 256 && uint64_t(nc) * (100 + n / 32) <= uint64_t(rate) * n; }
+
 void launch_reduce_bits(const uint32_t* bits, uint32_t nc, uint32_t nWords, uint32_t nDir, const float* N, const float* D, const float* W,
-                        int useCos, double* out, cudaStream_t st, double* w64) {
-  if (w64) {
+                        int useCos, double* out, cudaStream_t st, double* w64, bool plain) {
+  if (w64 && plain && warp_sums(nc, nDir, useCos ? 1500 : 1000)) {
+    if (useCos) launch_sum_warp<true>(BitsTerms<true>{bits, nc, N, D}, nDir, W, w64, out, st);
+    else launch_sum_warp<false>(BitsTerms<false>{bits, nc, N, D}, nDir, W, w64, out, st);
+  } else if (w64) {
     k_weights64<<<(nDir + 255) / 256, 256, 0, st>>>(W, nDir, w64);
-    k_reduce_bits_w64<<<(nc + kReduceBlock - 1) / kReduceBlock, kReduceBlock, 0, st>>>(bits, nc, nWords, N, D, w64, useCos, out);
+    k_reduce_bits_w64<<<blocks_of(nc), kReduceBlock, 0, st>>>(bits, nc, nWords, N, D, w64, useCos, out);
   } else if (nDir <= kReduceSmemDirs && reduce_smem_ready())
     k_reduce_bits<true><<<(nc + 255) / 256, 256, nDir * sizeof(double), st>>>(bits, nc, nWords, nDir, N, D, W, useCos, out);
   else k_reduce_bits<false><<<(nc + 255) / 256, 256, 0, st>>>(bits, nc, nWords, nDir, N, D, W, useCos, out);
 }
 void launch_reduce_bytes(const uint8_t* bytes, uint32_t nc, uint32_t nDir, const float* N, const float* D, const float* W, int useCos,
-                         double* out, cudaStream_t st, double* w64) {
-  if (w64) {
+                         double* out, cudaStream_t st, double* w64, bool plain) {
+  if (w64 && plain && warp_sums(nc, nDir, useCos ? 2500 : 2000)) {
+    if (useCos) launch_sum_warp<true>(BytesTerms<true>{bytes, nc, N, D}, nDir, W, w64, out, st);
+    else launch_sum_warp<false>(BytesTerms<false>{bytes, nc, N, D}, nDir, W, w64, out, st);
+  } else if (w64) {
     k_weights64<<<(nDir + 255) / 256, 256, 0, st>>>(W, nDir, w64);
-    k_reduce_bytes_w64<<<(nc + kReduceBlock - 1) / kReduceBlock, kReduceBlock, 0, st>>>(bytes, nc, nDir, N, D, w64, useCos, out);
+    k_reduce_bytes_w64<<<blocks_of(nc), kReduceBlock, 0, st>>>(bytes, nc, nDir, N, D, w64, useCos, out);
   } else if (nDir <= kReduceSmemDirs && reduce_smem_ready())
     k_reduce_bytes<true><<<(nc + 255) / 256, 256, nDir * sizeof(double), st>>>(bytes, nc, nDir, N, D, W, useCos, out);
   else k_reduce_bytes<false><<<(nc + 255) / 256, 256, 0, st>>>(bytes, nc, nDir, N, D, W, useCos, out);
 }
-void launch_reduce_dc(const float* dc, uint32_t nc, uint32_t nBins, const float* W, double* out, cudaStream_t st) {
-  k_reduce_dc<<<(nc + 255) / 256, 256, 0, st>>>(dc, nc, nBins, W, out);
+// sky bins: the warp form at every size (2306 bins, both forms, us a call: 500 sensors 673 / 48, 20,011 712 / 156,
+// 80,000 2005 / 868: two conversions and two FP64 operations a term against a rounded product)
+void launch_reduce_dc(const float* dc, uint32_t nc, uint32_t nBins, const float* W, double* out, cudaStream_t st, double* w64, bool plain) {
+  if (plain) launch_sum_warp<false>(DcTerms{dc, nc, nullptr}, nBins, W, w64, out, st);
+  else k_reduce_dc<<<(nc + 255) / 256, 256, 0, st>>>(dc, nc, nBins, W, out);
 }
 void launch_reduce_view(const ViewReduceArgs& a, cudaStream_t st) {
   // shared memory: per warp 2 C + R doubles and C floats per lane (at most 19 classes and 8 reach distances: 111 KB)
