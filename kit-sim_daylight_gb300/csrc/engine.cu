@@ -767,10 +767,8 @@ static int trace_impl(Engine& g, size_t i0, size_t nc, uint32_t rayFlags, uint64
   while (done < nc) {
     a.first = uint32_t(i0 + done); a.n = uint32_t(n); a.out0 = uint32_t(done); a.p0 = uint32_t(done);
     if (!reset_ctl(g)) return 0;
-    const size_t tasks = (n + 31) / 32 * g.nWords;   // warp tasks: 32 sensors x one 32-direction word
-    const int grid = int(std::min<size_t>(size_t(any ? g.gridBytes : g.gridBits), (tasks + 7) / 8));
     CU(cudaEventRecord(g.ev[0], g.st));
-    if (any) launch_bytes(a, grid, g.st); else launch_bits(a, grid, g.st, counters != nullptr);
+    if (any) launch_bytes(a, g.gridBytes, g.st); else launch_bits(a, g.gridBits, g.st, counters != nullptr);
     CU(cudaEventRecord(g.ev[1], g.st));
     if (!sync_status(g)) return 0;
     if (counters) {
@@ -1262,7 +1260,7 @@ KGB_API int kgb_view(kgb_engine* e, size_t i0, size_t nc, uint32_t rayFlags, con
   ViewArgs a{};
   a.nodes = static_cast<const Node8*>(g.sc->nodes.p); a.tris = static_cast<const TriRec*>(g.sc->tris.p); a.nNodes = walk_nodes(g);
   a.P = static_cast<const float*>(g.P.p); a.N = static_cast<const float*>(g.N.p);
-  a.stride = uint32_t(nc); a.i0 = uint32_t(i0); a.K = uint32_t(K); a.nWords = uint32_t(nWords); a.nAz = v->nAz; a.nEl = v->nEl;
+  a.stride = uint32_t(nc); a.i0 = uint32_t(i0); a.K = uint32_t(K); a.nAz = v->nAz; a.nEl = v->nEl;
   a.rayFlags = rayFlags; a.rowSin = static_cast<const float*>(g.rowSin.p); a.az0 = v->az0; a.dAz = v->dAz; a.groundZ = v->groundZ;
   a.cosN = float(std::cos(rad)); a.sinN = float(std::sin(rad));
   a.world = v->world ? 1 : 0; a.cull = v->cull ? 1 : 0; a.jitter = v->jitter ? 1 : 0; a.nS = v->nS; a.back = v->back ? 1 : 0;
@@ -1279,10 +1277,8 @@ KGB_API int kgb_view(kgb_engine* e, size_t i0, size_t nc, uint32_t rayFlags, con
     const size_t m = std::min(n, nc - done);
     a.first = uint32_t(i0 + done); a.n = uint32_t(m); a.out0 = uint32_t(done);
     if (!reset_ctl(g)) return 0;
-    const size_t tasks = (m + 31) / 32 * nWords;
-    const int grid = int(std::min<size_t>(size_t(g.gridView), (tasks + 7) / 8));
     CU(cudaEventRecord(g.ev[0], g.st));
-    launch_view(a, grid, g.st);
+    launch_view(a, g.gridView, g.st);
     CU(cudaEventRecord(g.ev[1], g.st));
     if (!sync_status(g)) return 0;
     const double ms = elapsed(g);

@@ -36,6 +36,7 @@ struct TraceArgs {
   const float* D;
   uint32_t first, n, out0, stride;
   uint32_t nDir, nWords, rayFlags;
+  uint32_t per;           // directions a task (set by launch_bytes)
   uint32_t* bits;
   uint8_t* bytes;
   const kgb_slot* slots;
@@ -61,7 +62,8 @@ struct ViewArgs {
   const float* P;
   const float* N;
   uint32_t first, n, out0, stride, i0;
-  uint32_t K, nWords, nAz, nEl, rayFlags;
+  uint32_t K, nAz, nEl, rayFlags;
+  uint32_t per;          // directions a task (set by launch_view)
   const float* rowSin;   // device [2 nEl]
   float az0, dAz, groundZ, cosN, sinN;
   uint32_t world, cull, jitter, nS, back, vground;
@@ -110,9 +112,10 @@ bool launch_rows(const void* in, size_t ld, void* out, size_t esize, uint32_t K,
 int bytes_blocks_per_sm();
 int view_blocks_per_sm();
 int bits_blocks_per_sm();
-void launch_bits(const TraceArgs& a, int grid, cudaStream_t st, bool count = false);
-void launch_bytes(const TraceArgs& a, int grid, cudaStream_t st);
-void launch_view(const ViewArgs& a, int grid, cudaStream_t st);
+// resident: the blocks the GPU holds at once (the grid is that or fewer)
+void launch_bits(const TraceArgs& a, int resident, cudaStream_t st, bool count = false);
+void launch_bytes(const TraceArgs& a, int resident, cudaStream_t st);
+void launch_view(const ViewArgs& a, int resident, cudaStream_t st);
 void launch_bounce(const BounceArgs& a, PathState* queues, uint32_t* qCount, int stepGrid, cudaStream_t st);
 size_t bounce_state_bytes();   // one queued path
 int bounce_step_blocks_per_sm();

@@ -517,17 +517,15 @@ __device__ __forceinline__ bool closest(const Scene& s, const Ray& r, float tmin
   }
 }
 
-// One visibility word: bit k = direction w*32+k of a sensor (normal n, ray origin o) passes the hemisphere cull and every
-// hit from tmin 1e-5 on is an own-plane hit, at most 3 (the reference's __raygen__bits, trace_dev.cu:91-108, restated
-// over the ray's hit set). COUNT adds traversal counters and rays traced.
+// Bits of one visibility word, those of directions d0 .. dEnd - 1: bit d % 32 = direction d of a sensor (normal n, ray
+// origin o) passes the hemisphere cull and every hit from tmin 1e-5 on is an own-plane hit, at most 3 (the reference's
+// __raygen__bits, trace_dev.cu:91-108, restated over the ray's hit set). COUNT adds traversal counters and rays traced.
 // tab: the directions' precomputed RayDir entries, or null (the rays are made from D).
 template <bool COUNT>
-__device__ __forceinline__ uint32_t trace_word(const Scene& s, F3 n, F3 o, const float* D, const RayDir* tab, uint32_t nDir, uint32_t w, bool cull,
-                                               uint32_t& overflow, Count& ctr, uint32_t& rays) {
+__device__ __forceinline__ uint32_t trace_word(const Scene& s, F3 n, F3 o, const float* D, const RayDir* tab, uint32_t d0, uint32_t dEnd,
+                                               bool cull, uint32_t& overflow, Count& ctr, uint32_t& rays) {
   uint32_t word = 0;
-  for (uint32_t k = 0; k < 32; ++k) {
-    const uint32_t d = w * 32 + k;
-    if (d >= nDir) break;
+  for (uint32_t d = d0; d < dEnd; ++d) {
     const F3 dir = ld3(D + 3 * d);
     if (!(n.x * dir.x + n.y * dir.y + n.z * dir.z > 0.f)) continue;
     const Ray r = tab ? ray_from(tab, d, o) : make_ray(o, dir);
@@ -539,7 +537,7 @@ __device__ __forceinline__ uint32_t trace_word(const Scene& s, F3 n, F3 o, const
       blocked = true;
       return true;
     }, overflow, &ctr);
-    if (!blocked) word |= 1u << k;
+    if (!blocked) word |= 1u << (d & 31u);
   }
   return word;
 }

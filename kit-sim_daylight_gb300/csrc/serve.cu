@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(256, 3) k_bits_batch(const BatchHdr* hdr, cons
     if (i >= g.n) continue;
     const Scene s{g.nodes, g.tris, g.nNodes};
     const F3 n = ld3(g.N + 3 * i), o = offset_ray(ld3(g.P + 3 * i), n);
-    const uint32_t word = trace_word<false>(s, n, o, g.D, g.tab, g.nDir, w, (g.rayFlags & KGB_RAY_CULL_BACK_FACING) != 0, overflow, ctr, rays);
+    const uint32_t word = trace_word<false>(s, n, o, g.D, g.tab, w * 32, min(w * 32 + 32, g.nDir), (g.rayFlags & KGB_RAY_CULL_BACK_FACING) != 0, overflow, ctr, rays);
     bitsPool[g.bitsOff + size_t(w) * g.n + i] = word;
   }
   if (overflow) atomicOr(status, (overflow & 1u ? kStatusStackOverflow : 0u) | (overflow & 2u ? kStatusVisitLimit : 0u));
@@ -606,7 +606,7 @@ bool launch_views(Server& s, int k, const Part& p, std::string& err) {
   a.nodes = static_cast<const Node8*>(sc.nodes); a.tris = static_cast<const TriRec*>(sc.tris); a.nNodes = sc.nNodes;
   a.P = reinterpret_cast<const float*>(b); a.N = reinterpret_cast<const float*>(b + L.offN);
   a.first = p.i0; a.n = p.n; a.out0 = 0; a.stride = p.n; a.i0 = p.i0;
-  a.K = uint32_t(K); a.nWords = uint32_t((K + 31) / 32); a.nAz = v.view.nAz; a.nEl = v.view.nEl; a.rayFlags = v.rayFlags;
+  a.K = uint32_t(K); a.nAz = v.view.nAz; a.nEl = v.view.nEl; a.rayFlags = v.rayFlags;
   a.rowSin = reinterpret_cast<const float*>(b + L.offRow); a.az0 = v.view.az0; a.dAz = v.view.dAz; a.groundZ = v.view.groundZ;
   a.cosN = float(std::cos(rad)); a.sinN = float(std::sin(rad));
   a.world = v.view.world ? 1 : 0; a.cull = v.view.cull ? 1 : 0; a.jitter = v.view.jitter ? 1 : 0; a.nS = v.view.nS; a.back = v.view.back ? 1 : 0;
@@ -623,11 +623,9 @@ bool launch_views(Server& s, int k, const Part& p, std::string& err) {
   ra.az0 = v.view.az0; ra.dAz = v.view.dAz; ra.rowSin = a.rowSin; ra.out = s.dViewOut;
   vs.part = p;
   vs.NA = ra.NA;
-  const size_t tasks = (size_t(p.n) + 31) / 32 * a.nWords;
-  const int grid = int(std::min<size_t>(size_t(s.gridView), (tasks + 7) / 8));
   if (!order_after_uploads(s, err) || !cuok(cudaEventRecord(vs.ev[0], s.st), err, "views") || !cuok(cudaMemsetAsync(vs.dCtl, 0, 8, s.st), err, "views"))
     return false;
-  launch_view(a, grid, s.st);
+  launch_view(a, s.gridView, s.st);
   launch_reduce_view(ra, s.st);
   return cuok(cudaGetLastError(), err, "views launch") &&
          cuok(cudaMemcpyAsync(vs.hOut, s.dViewOut, size_t(p.n) * ra.NA * 8, cudaMemcpyDeviceToHost, s.st), err, "views") &&

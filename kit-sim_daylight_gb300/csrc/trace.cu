@@ -5,12 +5,14 @@
 //  k_bounce_paths, k_bounce_step, k_bounce_accum
 //           reflected-light paths binned by sky patch (replaces __raygen__bounce, trace_dev.cu:260-311), as a wavefront
 //           of segments: first segments, then steps over a compacted queue of the paths that go on
-// The visibility kernels are persistent: each warp takes tasks of 32 consecutive sensors x one 32-direction word
-// from a global counter, so a warp traces one direction for 32 neighbouring sensors at a time (coherent rays). k_bits
+// The visibility kernels are persistent: each warp takes tasks of 32 consecutive sensors x up to 32 directions from a
+// global counter, so a warp traces one direction for 32 neighbouring sensors at a time (coherent rays). k_bits
 // and k_bytes take a call's sensors in the engine's tracing order (grouped by the orientation of their normals:
 // TraceArgs::order), so that a warp's sensors face the same way more often; each result goes to its sensor's column.
 #include "engine.h"
 #include "rt.cuh"
+
+#include <algorithm>
 
 namespace kgb {
 
@@ -36,24 +38,31 @@ __device__ __forceinline__ uint32_t next_task(uint32_t* counter) {
 
 // ---------------------------------------------------------------------------------------------------- bits
 // Direction d of a sensor is visible when n.d > 0 and every hit from tmin 1e-5 on is an own-plane hit, at most 3.
+// A task is 32 sensors x PER directions of a word (32, 16 or 8: task_directions; a template, since the whole word's form
+// keeps 80 registers without spills and the general one did not: 2 % of the urban trace).
 // COUNT: the instrumented variant (same results) that adds up nodes visited, triangles tested and rays traced.
-template <bool COUNT>
+template <bool COUNT, uint32_t PER>
 __global__ void __launch_bounds__(256) k_bits(TraceArgs a) {
   const Scene s{a.nodes, a.tris, a.nNodes};
   const bool cull = (a.rayFlags & KGB_RAY_CULL_BACK_FACING) != 0;
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t blocks = (a.n + 31) / 32, nTasks = blocks * a.nWords;
+  const uint32_t cols = a.nWords * (32 / PER), nTasks = (a.n + 31) / 32 * cols;
   uint32_t overflow = 0;
   Count ctr;
   uint32_t rays = 0;
   for (uint32_t task = next_task(a.counter); task < nTasks; task = next_task(a.counter)) {
-    const uint32_t b = task / a.nWords, w = task % a.nWords, i = b * 32 + lane;
+    const uint32_t i = task / cols * 32 + lane, d0 = task % cols * PER;
     if (i >= a.n) continue;
     uint32_t gi, col;
     task_sensor(a, i, gi, col);
     const F3 n = ld3(a.N + 3 * gi), o = offset_ray(ld3(a.P + 3 * gi), n);
-    const uint32_t word = trace_word<COUNT>(s, n, o, a.D, a.rayTab, a.nDir, w, cull, overflow, ctr, rays);
-    a.bits[size_t(w) * a.stride + col] = word;
+    const uint32_t word = trace_word<COUNT>(s, n, o, a.D, a.rayTab, d0, min(d0 + PER, a.nDir), cull, overflow, ctr, rays);
+    const uint32_t e0 = task % cols * PER;   // d0 again: not kept through the walks
+    uint32_t* out = a.bits + size_t(e0 / 32) * a.stride + col;
+    const uint32_t at = e0 % 32;
+    if (PER == 32) *out = word;
+    else if (PER == 16) reinterpret_cast<uint16_t*>(out)[at / 16] = uint16_t(word >> at);
+    else reinterpret_cast<uint8_t*>(out)[at / 8] = uint8_t(word >> at);
   }
   if (overflow) atomicOr(a.status, (overflow & 1u ? kStatusStackOverflow : 0u) | (overflow & 2u ? kStatusVisitLimit : 0u));
   if (COUNT) {
@@ -62,6 +71,30 @@ __global__ void __launch_bounds__(256) k_bits(TraceArgs a) {
     atomicAdd(c + 1, (unsigned long long)ctr.tris);
     atomicAdd(c + 2, (unsigned long long)rays);
   }
+}
+// A call of few words: a block per 32 sensors x a word, each of its 16 warps two of the directions. Where even tasks of 8
+// directions would not give every resident warp one, the call lasts as long as one task: 16 sensors x 4746 directions
+// 48 to 10 us, 16 x 15 22 to 8 us.
+constexpr uint32_t kFewWarps = 16;
+__global__ void __launch_bounds__(32 * kFewWarps) k_bits_few(TraceArgs a) {
+  __shared__ uint32_t words[32];
+  const Scene s{a.nodes, a.tris, a.nNodes};
+  const bool cull = (a.rayFlags & KGB_RAY_CULL_BACK_FACING) != 0;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x / 32, b = blockIdx.x / a.nWords, w = blockIdx.x % a.nWords, i = b * 32 + lane;
+  uint32_t overflow = 0, rays = 0, gi = 0, col = 0;
+  Count ctr;
+  if (warp == 0) words[lane] = 0;
+  __syncthreads();
+  if (i < a.n) {
+    task_sensor(a, i, gi, col);
+    const F3 n = ld3(a.N + 3 * gi), o = offset_ray(ld3(a.P + 3 * gi), n);
+    uint32_t word = 0;
+    for (uint32_t d = w * 32 + warp; d < min(w * 32 + 32, a.nDir); d += kFewWarps) word |= trace_word<false>(s, n, o, a.D, a.rayTab, d, d + 1, cull, overflow, ctr, rays);
+    if (word) atomicOr(&words[lane], word);
+  }
+  __syncthreads();
+  if (warp == 0 && i < a.n) a.bits[size_t(w) * a.stride + col] = words[lane];
+  if (overflow) atomicOr(a.status, (overflow & 1u ? kStatusStackOverflow : 0u) | (overflow & 2u ? kStatusVisitLimit : 0u));
 }
 
 // ---------------------------------------------------------------------------------------------------- bytes
@@ -143,16 +176,15 @@ __global__ void __launch_bounds__(256, 3) k_bytes(TraceArgs a) {   // 3 blocks a
   const Scene s{a.nodes, a.tris, a.nNodes};
   const bool cull = (a.rayFlags & KGB_RAY_CULL_BACK_FACING) != 0;
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t blocks = (a.n + 31) / 32, nTasks = blocks * a.nWords;
+  const uint32_t cols = (a.nDir + a.per - 1) / a.per, nTasks = (a.n + 31) / 32 * cols;
   uint32_t overflow = 0;
   for (uint32_t task = next_task(a.counter); task < nTasks; task = next_task(a.counter)) {
-    const uint32_t b = task / a.nWords, w = task % a.nWords, i = b * 32 + lane;
+    const uint32_t b = task / cols, d0 = task % cols * a.per, i = b * 32 + lane;
     if (i >= a.n) continue;
     uint32_t gi, col;
     task_sensor(a, i, gi, col);
     const F3 n = ld3(a.N + 3 * gi), o = offset_ray(ld3(a.P + 3 * gi), n);
-    for (uint32_t k = 0; k < 32; ++k) {
-      const uint32_t d = w * 32 + k;
+    for (uint32_t d = d0; d < d0 + a.per; ++d) {
       if (d >= a.nDir) break;
       a.bytes[size_t(d) * a.stride + col] = trace_byte(s, a, o, n, d, ld3(a.D + 3 * d), cull, overflow);
     }
@@ -196,11 +228,11 @@ __global__ void __launch_bounds__(256, 3) k_view(ViewArgs a) {   // 3 blocks an 
   const Scene s{a.nodes, a.tris, a.nNodes};
   const bool cull = (a.rayFlags & KGB_RAY_CULL_BACK_FACING) != 0;
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t blocks = (a.n + 31) / 32, nTasks = blocks * a.nWords;
+  const uint32_t cols = (a.K + a.per - 1) / a.per, nTasks = (a.n + 31) / 32 * cols;
   const float inf = __int_as_float(0x7f800000);
   uint32_t overflow = 0;
   for (uint32_t task = next_task(a.counter); task < nTasks; task = next_task(a.counter)) {
-    const uint32_t b = task / a.nWords, w = task % a.nWords, i = b * 32 + lane;
+    const uint32_t b = task / cols, d0 = task % cols * a.per, i = b * 32 + lane;
     if (i >= a.n) continue;
     const uint32_t gl = a.first + i;           // sensor within the engine's arrays
     const uint32_t gi = a.i0 + a.out0 + i;     // global sensor index (seeds)
@@ -219,8 +251,7 @@ __global__ void __launch_bounds__(256, 3) k_view(ViewArgs a) {   // 3 blocks an 
       }
       u = f3(r.y * f.z - r.z * f.y, r.z * f.x - r.x * f.z, r.x * f.y - r.y * f.x);
     }
-    for (uint32_t k = 0; k < 32; ++k) {
-      const uint32_t d = w * 32 + k;
+    for (uint32_t d = d0; d < d0 + a.per; ++d) {
       if (d >= a.K) break;
       const uint32_t col = d % a.nAz, row = d / a.nAz;
       const F3 l = view_cell(d, col, a.rowSin[2 * row], a.rowSin[2 * row + 1], a.az0, a.dAz, a.jitter != 0, element, side);
@@ -493,15 +524,43 @@ int view_blocks_per_sm() {   // resident blocks of k_view per SM
 }
 int bits_blocks_per_sm() {   // resident blocks of k_bits per SM (its persistent grid fills the GPU once)
   int b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_bits<false>, 256, 0) != cudaSuccess || b < 1) b = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_bits<false, 32>, 256, 0) != cudaSuccess || b < 1) b = 1;
   return b;
 }
-void launch_bits(const TraceArgs& a, int grid, cudaStream_t st, bool count) {
-  if (count) k_bits<true><<<grid, 256, 0, st>>>(a);
-  else k_bits<false><<<grid, 256, 0, st>>>(a);
+// Directions a task, for `sensors` blocks of 32 sensors x n directions on `warps` resident warps: 32, or fewer where the
+// tasks are so few that their uneven lengths (a task turned away from its directions is culled, one along a street walks
+// far) would leave warps idle at a launch's end: halved, down to `least`, until there are 64 tasks a warp. Kernel time
+// with 32 always / 16 / 32 / 64 / 256 tasks a warp: 20 k sensors x 9066 bytes 16.3 / 15.2 / 14.5 / 14.3 / 14.6 ms, 25 k x
+// 3600 views 23.2 / 21.6 / 20.9 / 20.6 / 20.7 ms, 12 k x 10,800 views 21.3 / 19.8 / 19.1 / 18.5 / 18.4 ms, 12 k x 2155
+// bits 1.84 / 1.55 / 1.54 / 1.54 / 1.55 ms.
+static uint32_t task_directions(size_t sensors, size_t n, size_t warps, uint32_t least) {
+  uint32_t per = 32;
+  while (per > least && sensors * ((n + per - 1) / per) < 64 * warps) per /= 2;
+  return per;
 }
-void launch_bytes(const TraceArgs& a, int grid, cudaStream_t st) { k_bytes<<<grid, 256, 0, st>>>(a); }
-void launch_view(const ViewArgs& a, int grid, cudaStream_t st) { k_view<<<grid, 256, 0, st>>>(a); }
+static int task_grid(size_t tasks, int resident) { return int(std::min<size_t>(size_t(resident), (tasks + 7) / 8)); }
+void launch_bits(const TraceArgs& a, int resident, cudaStream_t st, bool count) {
+  const size_t blocks = (size_t(a.n) + 31) / 32, words = blocks * a.nWords, warps = size_t(resident) * 8;
+  if (!count && 4 * words < warps) { k_bits_few<<<unsigned(words), 32 * kFewWarps, 0, st>>>(a); return; }
+  const uint32_t per = count ? 32u : task_directions(blocks, size_t(a.nWords) * 32, warps, 8);
+  const int grid = task_grid(words * (32 / per), resident);
+  if (count) k_bits<true, 32><<<grid, 256, 0, st>>>(a);
+  else if (per == 32) k_bits<false, 32><<<grid, 256, 0, st>>>(a);
+  else if (per == 16) k_bits<false, 16><<<grid, 256, 0, st>>>(a);
+  else k_bits<false, 8><<<grid, 256, 0, st>>>(a);
+}
+void launch_bytes(const TraceArgs& args, int resident, cudaStream_t st) {
+  TraceArgs a = args;
+  const size_t blocks = (size_t(a.n) + 31) / 32;
+  a.per = task_directions(blocks, a.nDir, size_t(resident) * 8, 1);
+  k_bytes<<<task_grid(blocks * ((a.nDir + a.per - 1) / a.per), resident), 256, 0, st>>>(a);
+}
+void launch_view(const ViewArgs& args, int resident, cudaStream_t st) {
+  ViewArgs a = args;
+  const size_t blocks = (size_t(a.n) + 31) / 32;
+  a.per = task_directions(blocks, a.K, size_t(resident) * 8, 1);
+  k_view<<<task_grid(blocks * ((size_t(a.K) + a.per - 1) / a.per), resident), 256, 0, st>>>(a);
+}
 // ln tn of each slot as a float pair (glass_TR's logarithm, once per slot; kgb_ln_pair, as kgb_powf takes it)
 __global__ void k_slot_logs(const kgb_slot* slots, uint32_t n, float2* out) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
