@@ -149,12 +149,13 @@ extern "C" void box_test_check(uint64_t seed, int kind, int nRays, uint64_t out[
       uint32_t prim, flags, slot;
       Hit h;
       load_tri(recs.data(), k, v0, v1, v2, prim, flags, slot);
-      if (!hit_tri(r, v0, v1, v2, 1e-5f, INFINITY, false, h)) continue;
+      if (!hit_vertices(r, v0, v1, v2, 1e-5f, INFINITY, false, h)) continue;
       all.push_back(prim);
       if (h.t < best || (h.t == best && prim < first)) { best = h.t; first = prim; }
     }
-    for_hits<false, false>(s, r, 1e-5f, INFINITY, false, [&](const Hit& h, F3, F3, F3, uint32_t, uint32_t) { walk.push_back(h.prim); return false; },
-                           overflow);
+    const auto note = [&](const Hit& h, F3, F3, F3, uint32_t, uint32_t) { walk.push_back(h.prim); return false; };
+    if (q % 2) for_hits<false, false>(s, r, 1e-5f, INFINITY, false, note, overflow);   // both forms of the triangle test
+    else for_hits<false, true>(s, r, 1e-5f, INFINITY, false, note, overflow);
     std::sort(all.begin(), all.end());
     std::sort(walk.begin(), walk.end());
     ClosestOut c;
