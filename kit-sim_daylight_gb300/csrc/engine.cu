@@ -302,6 +302,7 @@ struct Engine {
   size_t nLabel = 0;
   Buf scratch, out;
   Buf w64;           // a reduce's weights as doubles
+  Buf frontiers;     // a trace launch's frontiers, one per 32 sensors
   Buf ctl;   // [0] task counter, [1] status, [2..7] three u64 counters of the instrumented kernels
   bool ownStream = true;
   int seriesForm = 0;         // 0 split-BF16 tensor cores, 1 plain FP32
@@ -579,7 +580,7 @@ KGB_API void kgb_destroy(kgb_engine* e) {
   delete g->sc;
   for (DevMesh* m : g->meshes) delete m;
   for (Buf* b : {&g->slots, &g->P, &g->N, &g->D, &g->rayTab, &g->vis, &g->dc, &g->contrib, &g->viewCls, &g->viewDist, &g->rowSin, &g->label, &g->scratch, &g->out, &g->ctl,
-                 &g->vop, &g->sop, &g->csr, &g->sunCol, &g->rows, &g->border, &g->slotLog, &g->bq, &g->w64}) b->free();
+                 &g->vop, &g->sop, &g->csr, &g->sunCol, &g->rows, &g->border, &g->slotLog, &g->bq, &g->w64, &g->frontiers, &g->order, &g->cls, &g->clsFlags}) b->free();
   g->staging.free();
   for (cudaEvent_t ev : g->ev) if (ev) cudaEventDestroy(ev);
   for (cudaEvent_t ev : g->bandEv) if (ev) cudaEventDestroy(ev);
@@ -623,7 +624,7 @@ KGB_API int kgb_build(kgb_engine* e, const float* v, size_t nv, const uint32_t* 
 KGB_API void kgb_trim(kgb_engine* e, int sensors) {
   Engine& g = *E(e);
   cudaStreamSynchronize(g.st);
-  g.vis.free(); g.dc.free(); g.contrib.free(); g.scratch.free(); g.out.free(); g.w64.free(); g.viewCls.free(); g.viewDist.free();
+  g.vis.free(); g.frontiers.free(); g.dc.free(); g.contrib.free(); g.scratch.free(); g.out.free(); g.w64.free(); g.viewCls.free(); g.viewDist.free();
   g.vop.free(); g.sop.free(); g.csr.free(); g.sunCol.free();
   g.viewN = 0;
   if (sensors) {
@@ -766,6 +767,11 @@ static int trace_impl(Engine& g, size_t i0, size_t nc, uint32_t rayFlags, uint64
   }
   while (done < nc) {
     a.first = uint32_t(i0 + done); a.n = uint32_t(n); a.out0 = uint32_t(done); a.p0 = uint32_t(done);
+    a.frontiers = nullptr;
+    if (g.nDir >= kFrontierDirs && n * g.nDir >= kFrontierRays) {
+      if (!grow(g.frontiers, (n + 31) / 32 * frontier_bytes())) return 0;
+      a.frontiers = static_cast<FrontierRec*>(g.frontiers.p);
+    }
     if (!reset_ctl(g)) return 0;
     CU(cudaEventRecord(g.ev[0], g.st));
     if (any) launch_bytes(a, g.gridBytes, g.st); else launch_bits(a, g.gridBits, g.st, counters != nullptr);

@@ -76,6 +76,7 @@ __device__ __forceinline__ uint32_t find_seg(const Seg* segs, uint32_t nSegs, ui
 // Three blocks an SM, as k_bits: left to itself the compiler gives this kernel 100 registers and two blocks an SM, and
 // the batch's trace ran 13 % longer than the single-request kernel on the same rays.
 __global__ void __launch_bounds__(256, 3) k_bits_batch(const BatchHdr* hdr, const Seg* segs, uint32_t* bitsPool, uint32_t* counter, uint32_t* status) {
+  __shared__ Frontier frontier[8];
   const uint32_t nSegs = hdr->nSegs, nTasks = hdr->nTasks;
   const uint32_t lane = threadIdx.x & 31;
   uint32_t overflow = 0, rays = 0;
@@ -87,11 +88,20 @@ __global__ void __launch_bounds__(256, 3) k_bits_batch(const BatchHdr* hdr, cons
     if (task >= nTasks) break;
     const Seg& g = segs[find_seg(segs, nSegs, task, false)];
     const uint32_t local = task - g.taskBase, b = local / g.nWords, w = local % g.nWords, i = b * 32 + lane;
-    if (i >= g.n) continue;
+    const bool valid = i < g.n;
     const Scene s{g.nodes, g.tris, g.nNodes};
-    const F3 n = ld3(g.N + 3 * i), o = offset_ray(ld3(g.P + 3 * i), n);
-    const uint32_t word = trace_word<false>(s, n, o, g.D, g.tab, w * 32, min(w * 32 + 32, g.nDir), (g.rayFlags & KGB_RAY_CULL_BACK_FACING) != 0, overflow, ctr, rays);
-    bitsPool[g.bitsOff + size_t(w) * g.n + i] = word;
+    F3 n = f3(0.f, 0.f, 0.f), o = n;
+    if (valid) {
+      n = ld3(g.N + 3 * i);
+      o = offset_ray(ld3(g.P + 3 * i), n);
+    }
+    Frontier& f = frontier[threadIdx.x / 32];
+    const Bounds bounds = origin_bounds(o, valid);
+    const uint32_t entries = build_frontier(s, bounds, f, lane);
+    const uint32_t word = trace_word<false>(s, f, entries, bounds, n, o, valid, g.tab, w * 32, min(w * 32 + 32, g.nDir),
+                                            (g.rayFlags & KGB_RAY_CULL_BACK_FACING) != 0, overflow, ctr, rays);
+    __syncwarp();   // the frontier is the next task's
+    if (valid) bitsPool[g.bitsOff + size_t(w) * g.n + i] = word;
   }
   if (overflow) atomicOr(status, (overflow & 1u ? kStatusStackOverflow : 0u) | (overflow & 2u ? kStatusVisitLimit : 0u));
 }

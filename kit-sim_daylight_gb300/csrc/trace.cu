@@ -39,10 +39,12 @@ __device__ __forceinline__ uint32_t next_task(uint32_t* counter) {
 // ---------------------------------------------------------------------------------------------------- bits
 // Direction d of a sensor is visible when n.d > 0 and every hit from tmin 1e-5 on is an own-plane hit, at most 3.
 // A task is 32 sensors x PER directions of a word (32, 16 or 8: task_directions; a template, since the whole word's form
-// keeps 80 registers without spills and the general one did not: 2 % of the urban trace).
+// keeps 80 registers without spills and the general one did not: 2 % of the urban trace). FRONT: the walks start from the
+// 32 sensors' frontier (a.frontiers, by position in the launch), which k_frontiers made.
 // COUNT: the instrumented variant (same results) that adds up nodes visited, triangles tested and rays traced.
-template <bool COUNT, uint32_t PER>
+template <bool COUNT, uint32_t PER, bool FRONT>
 __global__ void __launch_bounds__(256) k_bits(TraceArgs a) {
+  __shared__ Frontier frontier[FRONT ? 8 : 1];
   const Scene s{a.nodes, a.tris, a.nNodes};
   const bool cull = (a.rayFlags & KGB_RAY_CULL_BACK_FACING) != 0;
   const uint32_t lane = threadIdx.x & 31;
@@ -52,11 +54,25 @@ __global__ void __launch_bounds__(256) k_bits(TraceArgs a) {
   uint32_t rays = 0;
   for (uint32_t task = next_task(a.counter); task < nTasks; task = next_task(a.counter)) {
     const uint32_t i = task / cols * 32 + lane, d0 = task % cols * PER;
-    if (i >= a.n) continue;
-    uint32_t gi, col;
-    task_sensor(a, i, gi, col);
-    const F3 n = ld3(a.N + 3 * gi), o = offset_ray(ld3(a.P + 3 * gi), n);
-    const uint32_t word = trace_word<COUNT>(s, n, o, a.D, a.rayTab, d0, min(d0 + PER, a.nDir), cull, overflow, ctr, rays);
+    const bool valid = i < a.n;
+    uint32_t gi = 0, col = 0, word = 0;
+    F3 n = f3(0.f, 0.f, 0.f), o = n;
+    if (valid) {
+      task_sensor(a, i, gi, col);
+      n = ld3(a.N + 3 * gi);
+      o = offset_ray(ld3(a.P + 3 * gi), n);
+    }
+    if (FRONT) {
+      const FrontierRec* rec = a.frontiers + task / cols;
+      Frontier& f = frontier[threadIdx.x / 32];
+      load_frontier(rec, f, lane);
+      const Bounds b = rec->b;
+      word = trace_word<COUNT>(s, f, rec->n, b, n, o, valid, a.rayTab, d0, min(d0 + PER, a.nDir), cull, overflow, ctr, rays);
+      __syncwarp();   // the frontier is the next task's
+    } else if (valid) {
+      word = trace_word<COUNT>(s, n, o, a.D, a.rayTab, d0, min(d0 + PER, a.nDir), cull, overflow, ctr, rays);
+    }
+    if (!valid) continue;
     const uint32_t e0 = task % cols * PER;   // d0 again: not kept through the walks
     uint32_t* out = a.bits + size_t(e0 / 32) * a.stride + col;
     const uint32_t at = e0 % 32;
@@ -71,6 +87,24 @@ __global__ void __launch_bounds__(256) k_bits(TraceArgs a) {
     atomicAdd(c + 1, (unsigned long long)ctr.tris);
     atomicAdd(c + 2, (unsigned long long)rays);
   }
+}
+// A launch's frontiers: a warp per 32 sensors.
+constexpr uint32_t kFrontierWarps = 4;
+__global__ void __launch_bounds__(32 * kFrontierWarps) k_frontiers(TraceArgs a) {
+  __shared__ Frontier frontier[kFrontierWarps];
+  const Scene s{a.nodes, a.tris, a.nNodes};
+  const uint32_t lane = threadIdx.x & 31, block = blockIdx.x * kFrontierWarps + threadIdx.x / 32, i = block * 32 + lane;
+  if (block * 32 >= a.n) return;   // whole warps
+  F3 o = f3(0.f, 0.f, 0.f);
+  if (i < a.n) {
+    uint32_t gi, col;
+    task_sensor(a, i, gi, col);
+    o = offset_ray(ld3(a.P + 3 * gi), ld3(a.N + 3 * gi));
+  }
+  Frontier& f = frontier[threadIdx.x / 32];
+  const Bounds b = origin_bounds(o, i < a.n);
+  const uint32_t n = build_frontier(s, b, f, lane);
+  store_frontier(a.frontiers + block, f, b, n, lane);
 }
 // A call of few words: a block per 32 sensors x a word, each of its 16 warps two of the directions. Where even tasks of 8
 // directions would not give every resident warp one, the call lasts as long as one task: 16 sensors x 4746 directions
@@ -89,7 +123,8 @@ __global__ void __launch_bounds__(32 * kFewWarps) k_bits_few(TraceArgs a) {
     task_sensor(a, i, gi, col);
     const F3 n = ld3(a.N + 3 * gi), o = offset_ray(ld3(a.P + 3 * gi), n);
     uint32_t word = 0;
-    for (uint32_t d = w * 32 + warp; d < min(w * 32 + 32, a.nDir); d += kFewWarps) word |= trace_word<false>(s, n, o, a.D, a.rayTab, d, d + 1, cull, overflow, ctr, rays);
+    for (uint32_t d = w * 32 + warp; d < min(w * 32 + 32, a.nDir); d += kFewWarps)
+      word |= trace_word<false>(s, n, o, a.D, a.rayTab, d, d + 1, cull, overflow, ctr, rays);
     if (word) atomicOr(&words[lane], word);
   }
   __syncthreads();
@@ -117,21 +152,20 @@ __device__ __forceinline__ float crossing(const kgb_slot* slots, const float2* s
 constexpr int kMaxCross = 16;   // translucent crossings a ray keeps in registers before it walks them in order instead
 
 // Own-plane hits pass (at most 3), an opaque hit blocks, translucent crossings multiply in (t, primitive) order.
-// d: the direction's index, whose precomputed ray part (a.rayTab, when set) gives the ray make_ray would.
-__device__ uint8_t trace_byte(const Scene& s, const TraceArgs& a, F3 o, F3 n, uint32_t d, F3 dir, bool cull, uint32_t& overflow) {
-  if (!(n.x * dir.x + n.y * dir.y + n.z * dir.z > 0.f)) return 0;
-  const Ray r = a.rayTab ? ray_from(a.rayTab, d, o) : make_ray(o, dir);
+// hits(f): calls f for every hit of the ray (origin's normal n, direction dir).
+template <class Hits>
+__device__ __forceinline__ uint8_t trace_byte(const TraceArgs& a, F3 n, F3 dir, Hits&& hits) {
   bool blocked = false, spill = false;
   int own = 0, nx = 0;
   float ct[kMaxCross], cf[kMaxCross];
   uint32_t cp[kMaxCross];
-  for_hits<false, true>(s, r, 1e-5f, INFINITY, cull, [&](const Hit& h, F3 v0, F3 v1, F3 v2, uint32_t flags, uint32_t slot) {
+  hits([&](const Hit& h, F3 v0, F3 v1, F3 v2, uint32_t flags, uint32_t slot) {
     if (own_hit(v0, v1, v2, h, dir, n)) { if (++own <= 3) return false; blocked = true; return true; }
     if (!(flags & kTriTranslucent)) { blocked = true; return true; }
     if (nx < kMaxCross) { ct[nx] = h.t; cp[nx] = h.prim; cf[nx] = crossing(a.slots, a.slotLog, a.nSlots, slot, h.front, v0, v1, v2, dir); ++nx; }
     else spill = true;
     return false;
-  }, overflow);
+  });
   if (blocked) return 0;
   float T = 1.f;
   if (!spill) {
@@ -155,7 +189,7 @@ __device__ uint8_t trace_byte(const Scene& s, const TraceArgs& a, F3 o, F3 n, ui
     bool found = false;
     float bt = 0.f, bf = 0.f;
     uint32_t bp = 0;
-    for_hits<false, true>(s, r, 1e-5f, INFINITY, cull, [&](const Hit& h, F3 v0, F3 v1, F3 v2, uint32_t flags, uint32_t slot) {
+    hits([&](const Hit& h, F3 v0, F3 v1, F3 v2, uint32_t flags, uint32_t slot) {
       if (!(flags & kTriTranslucent) || own_hit(v0, v1, v2, h, dir, n)) return false;
       if (h.t < lastT || (h.t == lastT && h.prim <= lastP)) return false;
       if (!found || h.t < bt || (h.t == bt && h.prim < bp)) {
@@ -163,7 +197,7 @@ __device__ uint8_t trace_byte(const Scene& s, const TraceArgs& a, F3 o, F3 n, ui
         bf = crossing(a.slots, a.slotLog, a.nSlots, slot, h.front, v0, v1, v2, dir);
       }
       return false;
-    }, overflow);
+    });
     if (!found) break;
     T *= bf;
     if (!(T >= 1.f / 510.f)) return 0;
@@ -172,22 +206,51 @@ __device__ uint8_t trace_byte(const Scene& s, const TraceArgs& a, F3 o, F3 n, ui
   return (uint8_t)__float2uint_rn(T * 255.f);
 }
 
+// FRONT: as k_bits.
+template <bool FRONT>
 __global__ void __launch_bounds__(256, 3) k_bytes(TraceArgs a) {   // 3 blocks an SM: 21.3 ms for a precision chunk, 24.6 at 2 (no spills)
+  __shared__ Frontier frontier[FRONT ? 8 : 1];
   const Scene s{a.nodes, a.tris, a.nNodes};
   const bool cull = (a.rayFlags & KGB_RAY_CULL_BACK_FACING) != 0;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t cols = (a.nDir + a.per - 1) / a.per, nTasks = (a.n + 31) / 32 * cols;
   uint32_t overflow = 0;
   for (uint32_t task = next_task(a.counter); task < nTasks; task = next_task(a.counter)) {
-    const uint32_t b = task / cols, d0 = task % cols * a.per, i = b * 32 + lane;
-    if (i >= a.n) continue;
-    uint32_t gi, col;
-    task_sensor(a, i, gi, col);
-    const F3 n = ld3(a.N + 3 * gi), o = offset_ray(ld3(a.P + 3 * gi), n);
-    for (uint32_t d = d0; d < d0 + a.per; ++d) {
-      if (d >= a.nDir) break;
-      a.bytes[size_t(d) * a.stride + col] = trace_byte(s, a, o, n, d, ld3(a.D + 3 * d), cull, overflow);
+    const uint32_t b = task / cols, d0 = task % cols * a.per, i = b * 32 + lane, dEnd = min(d0 + a.per, a.nDir);
+    const bool valid = i < a.n;
+    if (!FRONT && !valid) continue;
+    uint32_t gi = 0, col = 0;
+    F3 n = f3(0.f, 0.f, 0.f), o = n;
+    if (valid) {
+      task_sensor(a, i, gi, col);
+      n = ld3(a.N + 3 * gi);
+      o = offset_ray(ld3(a.P + 3 * gi), n);
     }
+    Frontier& f = frontier[FRONT ? threadIdx.x / 32 : 0];
+    uint32_t entries = 0;
+    Bounds bounds;
+    if (FRONT) {
+      const FrontierRec* rec = a.frontiers + b;
+      load_frontier(rec, f, lane);
+      bounds = rec->b;
+      entries = rec->n;
+    }
+    for (uint32_t d = d0; d < dEnd; ++d) {
+      const Ray r = ray_from(a.rayTab, d, o);
+      const bool on = n.x * r.d.x + n.y * r.d.y + n.z * r.d.z > 0.f;   // never for a lane without a sensor
+      uint8_t out = 0;
+      if (FRONT) {
+        if (__any_sync(~0u, on)) {
+          const Mask64 m = shaft(f, entries, bounds, r, lane);
+          if (on)
+            out = trace_byte(a, n, r.d, [&](auto&& hit) { frontier_hits<false, true>(s, f, m, r, 1e-5f, INFINITY, cull, hit, overflow, nullptr); });
+        }
+      } else if (on) {
+        out = trace_byte(a, n, r.d, [&](auto&& hit) { for_hits<false, true>(s, r, 1e-5f, INFINITY, cull, hit, overflow); });
+      }
+      if (valid) a.bytes[size_t(d) * a.stride + col] = out;
+    }
+    if (FRONT) __syncwarp();   // the frontier is the next task's
   }
   if (overflow) atomicOr(a.status, (overflow & 1u ? kStatusStackOverflow : 0u) | (overflow & 2u ? kStatusVisitLimit : 0u));
 }
@@ -514,7 +577,7 @@ void launch_ray_table(const float* D, uint32_t nDir, void* tab, cudaStream_t st)
 }
 int bytes_blocks_per_sm() {   // resident blocks of k_bytes per SM
   int b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_bytes, 256, 0) != cudaSuccess || b < 1) b = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_bytes<true>, 256, 0) != cudaSuccess || b < 1) b = 1;
   return b;
 }
 int view_blocks_per_sm() {   // resident blocks of k_view per SM
@@ -524,7 +587,7 @@ int view_blocks_per_sm() {   // resident blocks of k_view per SM
 }
 int bits_blocks_per_sm() {   // resident blocks of k_bits per SM (its persistent grid fills the GPU once)
   int b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_bits<false, 32>, 256, 0) != cudaSuccess || b < 1) b = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_bits<false, 32, true>, 256, 0) != cudaSuccess || b < 1) b = 1;
   return b;
 }
 // Directions a task, for `sensors` blocks of 32 sensors x n directions on `warps` resident warps: 32, or fewer where the
@@ -539,21 +602,31 @@ static uint32_t task_directions(size_t sensors, size_t n, size_t warps, uint32_t
   return per;
 }
 static int task_grid(size_t tasks, int resident) { return int(std::min<size_t>(size_t(resident), (tasks + 7) / 8)); }
+static void launch_frontiers(const TraceArgs& a, size_t blocks, cudaStream_t st) {
+  k_frontiers<<<unsigned((blocks + kFrontierWarps - 1) / kFrontierWarps), 32 * kFrontierWarps, 0, st>>>(a);
+}
 void launch_bits(const TraceArgs& a, int resident, cudaStream_t st, bool count) {
   const size_t blocks = (size_t(a.n) + 31) / 32, words = blocks * a.nWords, warps = size_t(resident) * 8;
   if (!count && 4 * words < warps) { k_bits_few<<<unsigned(words), 32 * kFewWarps, 0, st>>>(a); return; }
   const uint32_t per = count ? 32u : task_directions(blocks, size_t(a.nWords) * 32, warps, 8);
   const int grid = task_grid(words * (32 / per), resident);
-  if (count) k_bits<true, 32><<<grid, 256, 0, st>>>(a);
-  else if (per == 32) k_bits<false, 32><<<grid, 256, 0, st>>>(a);
-  else if (per == 16) k_bits<false, 16><<<grid, 256, 0, st>>>(a);
-  else k_bits<false, 8><<<grid, 256, 0, st>>>(a);
+  const bool front = a.frontiers != nullptr;
+  if (front) launch_frontiers(a, blocks, st);
+  if (count) front ? k_bits<true, 32, true><<<grid, 256, 0, st>>>(a) : k_bits<true, 32, false><<<grid, 256, 0, st>>>(a);
+  else if (per == 32) front ? k_bits<false, 32, true><<<grid, 256, 0, st>>>(a) : k_bits<false, 32, false><<<grid, 256, 0, st>>>(a);
+  else if (per == 16) front ? k_bits<false, 16, true><<<grid, 256, 0, st>>>(a) : k_bits<false, 16, false><<<grid, 256, 0, st>>>(a);
+  else front ? k_bits<false, 8, true><<<grid, 256, 0, st>>>(a) : k_bits<false, 8, false><<<grid, 256, 0, st>>>(a);
 }
+size_t frontier_bytes() { return sizeof(FrontierRec); }
 void launch_bytes(const TraceArgs& args, int resident, cudaStream_t st) {
   TraceArgs a = args;
   const size_t blocks = (size_t(a.n) + 31) / 32;
   a.per = task_directions(blocks, a.nDir, size_t(resident) * 8, 1);
-  k_bytes<<<task_grid(blocks * ((a.nDir + a.per - 1) / a.per), resident), 256, 0, st>>>(a);
+  const int grid = task_grid(blocks * ((a.nDir + a.per - 1) / a.per), resident);
+  if (a.frontiers) {
+    launch_frontiers(a, blocks, st);
+    k_bytes<true><<<grid, 256, 0, st>>>(a);
+  } else k_bytes<false><<<grid, 256, 0, st>>>(a);
 }
 void launch_view(const ViewArgs& args, int resident, cudaStream_t st) {
   ViewArgs a = args;
