@@ -273,6 +273,11 @@ struct SceneObj {
 // 17.74 / 18.36 / 18.13e9 sensor-steps/s (at 8 the shorter launches' tails cost more kernel time than they save).
 constexpr uint32_t kSeriesBands = 6;
 
+constexpr size_t kSmallAt = 256, kSmallBytes = size_t(64) << 10;   // a reduce's weights and its sums, if each fits
+// Sensors from which on set_scene orders them by orientation (below, a warp's worth or a few, the order's kernel, its
+// wait and its copy back cost more than the trace saves: 16 sensors, 20 us of 98).
+constexpr size_t kOrderSensors = 1024;
+
 struct Engine {
   int device = 0, numSMs = 0;
   cudaStream_t st = nullptr;
@@ -285,6 +290,7 @@ struct Engine {
   Buf order;                          // the sensors grouped by normal orientation (TraceArgs::order), on the device
   std::vector<uint32_t> orderHost;    // and here, to find a call's runs
   uint32_t classStart[7] = {};        // class c's sensors are orderHost[classStart[c] .. classStart[c + 1])
+  bool ordered = false;               // order and the rest are the present sensors'
   Buf cls, clsFlags;                  // the classes the order was built from (a byte per sensor); the class kernel's flags
   Buf vis;
   bool bytes = false;
@@ -304,6 +310,10 @@ struct Engine {
   Buf w64;           // a reduce's weights as doubles
   Buf frontiers;     // a trace launch's frontiers, one per 32 sensors
   Buf ctl;   // [0] task counter, [1] status, [2..7] three u64 counters of the instrumented kernels
+  // Page-locked host memory that kernels read and write in place (the host's and the GPU's memory are one address space, and
+  // a small copy costs more than the few lines it moves): [0] the status word of the visibility kernels, [1..7] the sensor
+  // classes' flags, from kSmallAt on a small reduce's weights, then its sums. Used within a call, which waits for its work.
+  uint32_t* host = nullptr;
   bool ownStream = true;
   int seriesForm = 0;         // 0 split-BF16 tensor cores, 1 plain FP32
   Buf vop, sop, csr, sunCol;
@@ -358,11 +368,12 @@ int download_rows(Engine& g, const void* dev, size_t esize, size_t K, size_t nc,
   return download_rows_into(g.rows, g.staging, dev, esize, K, nc, host, g.st);
 }
 
-int sync_status(Engine& g) {   // wait for the stream, then read the kernels' status word
+int sync_status(Engine& g, bool inHost) {   // wait for the stream, then read the kernels' status word (in g.host, or in g.ctl)
   uint32_t status = 0;
-  CU(cudaMemcpyAsync(&status, static_cast<uint32_t*>(g.ctl.p) + 1, 4, cudaMemcpyDeviceToHost, g.st));
+  if (!inHost) CU(cudaMemcpyAsync(&status, static_cast<uint32_t*>(g.ctl.p) + 1, 4, cudaMemcpyDeviceToHost, g.st));
   CU(cudaStreamSynchronize(g.st));
   CU(cudaGetLastError());
+  if (inHost) status = *static_cast<volatile uint32_t*>(g.host);
   if (status & kStatusStackOverflow) return fail("traversal stack overflow (BVH deeper than the kernel's stack)");
   if (status & kStatusVisitLimit)
     return fail("traversal gave up: a query passed its node-visit limit (the BVH's node count + 8, at most 2^20) or met a node index beyond the BVH");
@@ -567,6 +578,7 @@ KGB_API kgb_engine* kgb_init(void) {
   if (cudaStreamCreateWithFlags(&g->st, cudaStreamNonBlocking) != cudaSuccess) return bad("cudaStreamCreate failed");
   if (cudaEventCreate(&g->ev[0]) != cudaSuccess || cudaEventCreate(&g->ev[1]) != cudaSuccess) return bad("cudaEventCreate failed");
   if (!grow(g->ctl, 128)) return bad(g_err);
+  if (cudaHostAlloc(reinterpret_cast<void**>(&g->host), kSmallAt + 2 * kSmallBytes, cudaHostAllocMapped) != cudaSuccess) return bad("cudaHostAlloc failed");
   g->sc = new SceneObj;
   const kgb_slot one{0.2f, 0.f, 0.f, 0u};
   if (!kgb_set_slots(reinterpret_cast<kgb_engine*>(g), &one, 1)) return bad(g_err);
@@ -582,6 +594,7 @@ KGB_API void kgb_destroy(kgb_engine* e) {
   for (Buf* b : {&g->slots, &g->P, &g->N, &g->D, &g->rayTab, &g->vis, &g->dc, &g->contrib, &g->viewCls, &g->viewDist, &g->rowSin, &g->label, &g->scratch, &g->out, &g->ctl,
                  &g->vop, &g->sop, &g->csr, &g->sunCol, &g->rows, &g->border, &g->slotLog, &g->bq, &g->w64, &g->frontiers, &g->order, &g->cls, &g->clsFlags}) b->free();
   g->staging.free();
+  if (g->host) cudaFreeHost(g->host);
   for (cudaEvent_t ev : g->ev) if (ev) cudaEventDestroy(ev);
   for (cudaEvent_t ev : g->bandEv) if (ev) cudaEventDestroy(ev);
   if (g->copySt) { cudaStreamSynchronize(g->copySt); cudaStreamDestroy(g->copySt); }
@@ -630,6 +643,7 @@ KGB_API void kgb_trim(kgb_engine* e, int sensors) {
   if (sensors) {
     g.P.free(); g.N.free(); g.label.free(); g.order.free(); g.cls.free(); g.nLabel = 0; g.nSensors = 0;
     std::vector<uint32_t>().swap(g.orderHost);
+    g.ordered = false;
   }
 }
 
@@ -678,16 +692,22 @@ KGB_API uint64_t kgb_free_bytes(void) {
 // same rays, so the order is rebuilt only when the classes of the sensors just uploaded differ from those it was built
 // from (a kernel compares them on the device; a caller that sends the same sensors every step pays for that kernel).
 static bool sensor_order(Engine& g, size_t nSensors) {
-  const bool fresh = g.orderHost.size() != nSensors || !g.order.p;
+  if (nSensors < kOrderSensors) {   // none: the traces take them as they come
+    g.orderHost.clear();
+    g.ordered = false;
+    return true;
+  }
+  const bool fresh = !g.ordered || g.orderHost.size() != nSensors || !g.order.p;
+  g.ordered = true;
   if (!grow(g.cls, nSensors) || !grow(g.clsFlags, 7 * 4)) return false;
-  if (fresh && nSensors) CU(cudaMemsetAsync(g.cls.p, 0xff, nSensors, g.st));   // no class yet: every sensor differs
+  if (fresh) CU(cudaMemsetAsync(g.cls.p, 0xff, nSensors, g.st));   // no class yet: every sensor differs
   CU(cudaMemsetAsync(g.clsFlags.p, 0, 7 * 4, g.st));
   launch_sensor_classes(static_cast<const float*>(g.N.p), uint32_t(nSensors), static_cast<uint8_t*>(g.cls.p),
                         static_cast<uint32_t*>(g.clsFlags.p), g.st);
   CU(cudaGetLastError());
-  uint32_t f[7];
-  CU(cudaMemcpyAsync(f, g.clsFlags.p, sizeof f, cudaMemcpyDeviceToHost, g.st));
+  CU(cudaMemcpyAsync(g.host + 1, g.clsFlags.p, 7 * 4, cudaMemcpyDeviceToHost, g.st));
   CU(cudaStreamSynchronize(g.st));
+  const uint32_t* f = g.host + 1;
   if (!f[0] && !fresh) return true;
   std::vector<uint8_t> cls(nSensors);
   if (nSensors) {
@@ -749,9 +769,10 @@ static int trace_impl(Engine& g, size_t i0, size_t nc, uint32_t rayFlags, uint64
   a.bits = any ? nullptr : static_cast<uint32_t*>(g.vis.p);
   a.bytes = any ? static_cast<uint8_t*>(g.vis.p) : nullptr;
   a.slots = static_cast<const kgb_slot*>(g.slots.p); a.nSlots = g.nSlots; a.slotLog = static_cast<const float2*>(g.slotLog.p);
-  a.counter = static_cast<uint32_t*>(g.ctl.p); a.status = static_cast<uint32_t*>(g.ctl.p) + 1;
+  a.counter = static_cast<uint32_t*>(g.ctl.p); a.status = counters ? static_cast<uint32_t*>(g.ctl.p) + 1 : g.host;
+  g.host[0] = 0;
   a.rayTab = static_cast<const RayDir*>(g.rayTab.p);
-  if (g.orderHost.size() == g.nSensors) {   // the call's range in tracing order: per class, its run of the order
+  if (g.ordered) {   // the call's range in tracing order: per class, its run of the order
     a.order = static_cast<const uint32_t*>(g.order.p);
     a.callI0 = uint32_t(i0);
     uint32_t end = 0;
@@ -776,7 +797,7 @@ static int trace_impl(Engine& g, size_t i0, size_t nc, uint32_t rayFlags, uint64
     CU(cudaEventRecord(g.ev[0], g.st));
     if (any) launch_bytes(a, g.gridBytes, g.st); else launch_bits(a, g.gridBits, g.st, counters != nullptr);
     CU(cudaEventRecord(g.ev[1], g.st));
-    if (!sync_status(g)) return 0;
+    if (!sync_status(g, !counters)) return 0;
     if (counters) {
       uint64_t c[3];
       CU(cudaMemcpy(c, static_cast<uint32_t*>(g.ctl.p) + 2, sizeof c, cudaMemcpyDeviceToHost));
@@ -811,22 +832,49 @@ KGB_API int kgb_set_stream(kgb_engine* e, void* stream) {
   return 1;
 }
 
+// Where a reduce's kernels read its n weights and write its sums: in the engine's page-locked memory where they fit, else on
+// the device, the weights copied there. A box's reduce spent 16 us of 27 in its two copies.
+static int reduce_ends(Engine& g, const float* W, size_t n, size_t nc, const float** w, double** sums) {
+  char* small = reinterpret_cast<char*>(g.host) + kSmallAt;
+  if (n * 4 <= kSmallBytes) {
+    if (n) std::memcpy(small, W, n * 4);
+    *w = reinterpret_cast<const float*>(small);
+  } else {
+    if (!upload(g.scratch, W, n * 4, g.st)) return 0;
+    *w = static_cast<const float*>(g.scratch.p);
+  }
+  if (nc * 8 <= kSmallBytes) *sums = reinterpret_cast<double*>(small + kSmallBytes);
+  else {
+    if (!grow(g.out, nc * 8)) return 0;
+    *sums = static_cast<double*>(g.out.p);
+  }
+  return 1;
+}
+static int reduce_done(Engine& g, size_t nc, const double* sums, double* out) {
+  CU(cudaGetLastError());
+  const bool small = nc * 8 <= kSmallBytes;
+  if (!small) CU(cudaMemcpyAsync(out, sums, nc * 8, cudaMemcpyDeviceToHost, g.st));
+  CU(cudaStreamSynchronize(g.st));
+  if (small) std::memcpy(out, sums, nc * 8);
+  return 1;
+}
+
 KGB_API int kgb_reduce(kgb_engine* e, size_t nc, const float* W, int useCos, double* out) {
   Engine& g = *E(e);
   if (nc == 0) return 1;
   if (nc != g.visN) return fail("gpu_reduce: no trace of this chunk");
-  if (!upload(g.scratch, W, g.nDir * 4, g.st) || !grow(g.out, nc * 8) || !grow(g.w64, g.nDir * 8)) return 0;
+  if (!grow(g.w64, g.nDir * 8)) return 0;
+  const float* w = nullptr;
+  double* sums = nullptr;
+  if (!reduce_ends(g, W, g.nDir, nc, &w, &sums)) return 0;
   const float* N = static_cast<const float*>(g.N.p) + 3 * g.i0;
   double* w64 = static_cast<double*>(g.w64.p);
   const bool plain = plain_weights(W, g.nDir);
-  if (g.bytes) launch_reduce_bytes(static_cast<const uint8_t*>(g.vis.p), uint32_t(nc), uint32_t(g.nDir), N, static_cast<const float*>(g.D.p),
-                                   static_cast<const float*>(g.scratch.p), useCos, static_cast<double*>(g.out.p), g.st, w64, plain);
-  else launch_reduce_bits(static_cast<const uint32_t*>(g.vis.p), uint32_t(nc), uint32_t(g.nWords), uint32_t(g.nDir), N, static_cast<const float*>(g.D.p),
-                          static_cast<const float*>(g.scratch.p), useCos, static_cast<double*>(g.out.p), g.st, w64, plain);
-  CU(cudaGetLastError());
-  CU(cudaMemcpyAsync(out, g.out.p, nc * 8, cudaMemcpyDeviceToHost, g.st));
-  CU(cudaStreamSynchronize(g.st));
-  return 1;
+  if (g.bytes) launch_reduce_bytes(static_cast<const uint8_t*>(g.vis.p), uint32_t(nc), uint32_t(g.nDir), N, static_cast<const float*>(g.D.p), w, useCos, sums,
+                                   g.st, w64, plain);
+  else launch_reduce_bits(static_cast<const uint32_t*>(g.vis.p), uint32_t(nc), uint32_t(g.nWords), uint32_t(g.nDir), N, static_cast<const float*>(g.D.p), w,
+                          useCos, sums, g.st, w64, plain);
+  return reduce_done(g, nc, sums, out);
 }
 
 namespace kgb {
@@ -1203,7 +1251,7 @@ KGB_API int kgb_bounce(kgb_engine* e, size_t i0, size_t nc, uint32_t rayFlags, c
     }
     if (ctl[1] & kStatusVisitLimit)
       return fail("gpu_bounce: traversal gave up (a walk passed its node-visit limit, or met a node index beyond the BVH)" + where);
-    if (!sync_status(g)) return 0;
+    if (!sync_status(g, false)) return 0;
     const double ms = elapsed(g);
     g.stats.bounceMs += ms; g.stats.paths += n * nc; g.stats.bounceLaunches++;
     done += n;
@@ -1217,13 +1265,12 @@ KGB_API int kgb_reduce_dc(kgb_engine* e, size_t nc, const float* W, double* out)
   Engine& g = *E(e);
   if (nc == 0) return 1;
   if (nc != g.dcN) return fail("gpu_reduce_dc: no gpu_bounce rows for this chunk");
-  if (!upload(g.scratch, W, g.nBins * 4, g.st) || !grow(g.out, nc * 8) || !grow(g.w64, g.nBins * 8)) return 0;
-  launch_reduce_dc(static_cast<const float*>(g.dc.p), uint32_t(nc), uint32_t(g.nBins), static_cast<const float*>(g.scratch.p), static_cast<double*>(g.out.p),
-                   g.st, static_cast<double*>(g.w64.p), plain_weights(W, g.nBins));
-  CU(cudaGetLastError());
-  CU(cudaMemcpyAsync(out, g.out.p, nc * 8, cudaMemcpyDeviceToHost, g.st));
-  CU(cudaStreamSynchronize(g.st));
-  return 1;
+  if (!grow(g.w64, g.nBins * 8)) return 0;
+  const float* w = nullptr;
+  double* sums = nullptr;
+  if (!reduce_ends(g, W, g.nBins, nc, &w, &sums)) return 0;
+  launch_reduce_dc(static_cast<const float*>(g.dc.p), uint32_t(nc), uint32_t(g.nBins), w, sums, g.st, static_cast<double*>(g.w64.p), plain_weights(W, g.nBins));
+  return reduce_done(g, nc, sums, out);
 }
 
 KGB_API int kgb_download_dc(kgb_engine* e, size_t nc, float* out, size_t count) {
@@ -1273,7 +1320,8 @@ KGB_API int kgb_view(kgb_engine* e, size_t i0, size_t nc, uint32_t rayFlags, con
   a.vground = v->vground ? 1 : 0;
   a.label = g.nLabel ? static_cast<const uint8_t*>(g.label.p) : nullptr;
   a.cls = static_cast<uint8_t*>(g.viewCls.p); a.dist = static_cast<float*>(g.viewDist.p);
-  a.counter = static_cast<uint32_t*>(g.ctl.p); a.status = static_cast<uint32_t*>(g.ctl.p) + 1;
+  a.counter = static_cast<uint32_t*>(g.ctl.p); a.status = g.host;
+  g.host[0] = 0;
   // gpu.cu:590: sub-launches of at least 2^13 threads there; here at least four (32 sensors x word) tasks for each
   // resident warp, so that no launch leaves the GPU idle; then ~40 ms, at most doubling, as the reference
   const size_t nMin = std::max<size_t>((size_t(1) << 13) / nWords, (size_t(4) * g.gridView * 8 * 32 + nWords - 1) / nWords);
@@ -1286,7 +1334,7 @@ KGB_API int kgb_view(kgb_engine* e, size_t i0, size_t nc, uint32_t rayFlags, con
     CU(cudaEventRecord(g.ev[0], g.st));
     launch_view(a, g.gridView, g.st);
     CU(cudaEventRecord(g.ev[1], g.st));
-    if (!sync_status(g)) return 0;
+    if (!sync_status(g, true)) return 0;
     const double ms = elapsed(g);
     g.stats.traceMs += ms; g.stats.rays += m * K; g.stats.launches++;
     done += m;
