@@ -405,10 +405,10 @@ __global__ void __launch_bounds__(32 * kSumWarps) k_sum_warp(S t, uint32_t n, co
   const F3 v = t.sensor(i);
   OrderedSum s;
   bool odd = false;
-  for (uint32_t d0 = 0; d0 < n; d0 += 32 * kAhead) {
-    typename S::Raw raw[kAhead];
-    F3 dir[kAhead];
-    uint2 w[kAhead];
+  typename S::Raw raw[kAhead];
+  F3 dir[kAhead];
+  uint2 w[kAhead];
+  const auto read = [&](uint32_t d0) {
 #pragma unroll
     for (int k = 0; k < kAhead; ++k) {
       const uint32_t d = min(d0 + 32 * k + lane, n - 1);
@@ -416,14 +416,19 @@ __global__ void __launch_bounds__(32 * kSumWarps) k_sum_warp(S t, uint32_t n, co
       if (COS) dir[k] = ld3(t.D + 3 * d);
       w[k] = __ldg(W + d);
     }
+  };
+  read(0);
+  for (uint32_t d0 = 0; d0 < n; d0 += 32 * kAhead) {
+    uint64_t p[kAhead];
+    int32_t e[kAhead];
 #pragma unroll
     for (int k = 0; k < kAhead; ++k) {
       const uint32_t d = d0 + 32 * k + lane;
-      uint64_t p;
-      int32_t e;
-      term(d < n ? t.factor(raw[k], d, cosine<COS>(v, dir[k])) : 0.f, w[k], p, e, odd);
-      add_32(s, p, e, lane);
+      term(d < n ? t.factor(raw[k], d, cosine<COS>(v, dir[k])) : 0.f, w[k], p[k], e[k], odd);
     }
+    if (d0 + 32 * kAhead < n) read(d0 + 32 * kAhead);   // under way while these are added
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) add_32(s, p[k], e[k], lane);
   }
   odd = __any_sync(~0u, odd);
   if (lane) return;
