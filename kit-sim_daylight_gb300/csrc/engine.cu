@@ -274,9 +274,11 @@ struct SceneObj {
 constexpr uint32_t kSeriesBands = 6;
 
 constexpr size_t kSmallAt = 256, kSmallBytes = size_t(64) << 10;   // a reduce's weights and its sums, if each fits
-// Sensors from which on set_scene orders them by orientation (below, a warp's worth or a few, the order's kernel, its
-// wait and its copy back cost more than the trace saves: 16 sensors, 20 us of 98).
-constexpr size_t kOrderSensors = 1024;
+// Sensors, and sensors x directions, from which on set_scene orders the sensors by orientation: a warp's worth gains
+// nothing, and a trace of few rays less than the 20 us of the order's kernel, wait and copy back (16 sensors x 15
+// directions: 20 us of 98; 1000 x 790: 178 us with the order, 168 without; 1000 x 5610: the trace takes 0.41 ms with it, 0.53
+// without).
+constexpr size_t kOrderSensors = 33, kOrderRays = size_t(1) << 20;
 
 struct Engine {
   int device = 0, numSMs = 0;
@@ -692,7 +694,7 @@ KGB_API uint64_t kgb_free_bytes(void) {
 // same rays, so the order is rebuilt only when the classes of the sensors just uploaded differ from those it was built
 // from (a kernel compares them on the device; a caller that sends the same sensors every step pays for that kernel).
 static bool sensor_order(Engine& g, size_t nSensors) {
-  if (nSensors < kOrderSensors) {   // none: the traces take them as they come
+  if (nSensors < kOrderSensors || nSensors * g.nDir < kOrderRays) {   // none: the traces take them as they come
     g.orderHost.clear();
     g.ordered = false;
     return true;
