@@ -268,10 +268,34 @@ struct SceneObj {
 
 }  // namespace
 
-// Bands of a chunk's series whose downloads overlap the next band's kernel; the first band's kernel and the last band's
-// download are not overlapped. Precision config (29,609-sensor chunks, E returned to host memory): 4 / 6 / 8 bands gave
-// 17.74 / 18.36 / 18.13e9 sensor-steps/s (at 8 the shorter launches' tails cost more kernel time than they save).
+// Bands of a chunk's series, whose downloads overlap the next band's kernel (the first band's kernel and the last band's
+// download overlap nothing): the count, up to six, whose pipeline ends first. A launch's 128 x 64 tiles run one to an SM
+// and its last round waits for all of them, so a band takes its rounds times a tile's time. The constants are the
+// contraction's rate an SM, a launch's start, the link's rate and a download's start, as measured. 29,609 sensors x 4456
+// steps, K 4672: 4 / 6 / 8 bands gave 17.74 / 18.36 / 18.13e9 sensor-steps/s, K 2368: 6 / 8 bands 4.18 / 4.22 ms.
+// Against six bands from 48 tile rows on and one below: 5000 sensors x 4456 steps 1573 to 1265 us with five bands, 8200
+// sensors 1720 to 1630 us with five (30 rounds of tiles where six bands are 36).
 constexpr uint32_t kSeriesBands = 6;
+constexpr double kTileRate = 1.02e13, kBandLaunch = 6e-6, kDownRate = 1.9e11, kDownStart = 2e-5;
+
+// rows of 128 sensors to a band
+inline uint32_t series_band_rows(uint32_t rows, uint64_t T, uint64_t Kp, uint32_t sms) {
+  const uint32_t nT = uint32_t((T + 63) / 64);
+  const double round = 128. * 64 * 12 * double(Kp) / kTileRate, down = 128. * double(T) * 4 / kDownRate;   // six products
+  uint32_t best = rows;
+  double bestEnd = 0;
+  for (uint32_t bands = 1; bands <= kSeriesBands && bands <= rows; ++bands) {
+    const uint32_t per = (rows + bands - 1) / bands;
+    double ran = 0, end = 0;
+    for (uint32_t r = 0; r < rows; r += per) {
+      const uint32_t m = std::min(per, rows - r);
+      ran += kBandLaunch + round * double((uint64_t(m) * nT + sms - 1) / sms);
+      end = std::max(end, ran) + kDownStart + down * m;
+    }
+    if (bands == 1 || end < bestEnd) { best = per; bestEnd = end; }
+  }
+  return best;
+}
 
 constexpr size_t kSmallAt = 256, kSmallBytes = size_t(64) << 10;   // a reduce's weights and its sums, if each fits
 // Sensors, and sensors x directions, from which on set_scene orders the sensors by orientation: a warp's worth gains
@@ -956,7 +980,8 @@ static int series_impl(Engine& g, size_t nc, const kgb_series_in* in, const Sink
     // E in bands of sensor rows: every band's kernel is queued on the engine's stream, and each band's rows go down
     // on the copy stream once its kernel is done, beside the next band's kernel (the first band's event also orders
     // the copies after this call's uploads, which used the same staging slices)
-    const uint32_t mAll = uint32_t((nc + 127) / 128), bands = mAll >= 8 * kSeriesBands ? kSeriesBands : 1, per = (mAll + bands - 1) / bands;
+    const uint32_t mAll = uint32_t((nc + 127) / 128), per = series_band_rows(mAll, T, Kp, uint32_t(g.numSMs)),
+                   bands = (mAll + per - 1) / per;
     if (!g.copySt) CU(cudaStreamCreateWithFlags(&g.copySt, cudaStreamNonBlocking));
     CU(cudaEventRecord(g.ev[0], g.st));
     for (uint32_t b = 0; b < bands; ++b) {
