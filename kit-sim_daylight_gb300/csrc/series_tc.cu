@@ -403,11 +403,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_series_tc(const __grid_constant_
 
 // The sun term of the reference's k_series tail (gpu.cu:145-148), added to E after the contraction: for column t with a
 // sun direction j (sunOfCol), E[i, t] + max(0, N_i . sun_j) at(i, sun0 + j) w_j when the sensor's visibility at of it
-// is not zero, in float with the reference's operation order. A block covers 32 sensors x 64 columns: the terms are
-// computed with lanes over sensors (the visibility reads coalesce) and added with lanes over columns (the E reads and
-// writes coalesce), through shared memory.
-constexpr uint32_t kSunRows = 32, kSunCols = 64;
-constexpr uint32_t kNoTerm = 0xffffffffu;   // no sun term (a NaN pattern the term's arithmetic does not produce on the GPU)
+// is not zero, in float with the reference's operation order. A warp covers 16 sensors x 32 columns, a lane a column:
+// E's rows coalesce, consecutive columns' visibility words are mostly one word (and one sector holds eight rows'), and
+// nothing passes through shared memory. It is bound by E's read and write in L2. Against terms computed with lanes over
+// sensors and turned through shared memory: the series kernels of 8200 sensors x 4456 steps 897 to 840 us (the call 1630
+// to 1595 us), of 29,609 with reflected light 5.26 to 5.09 ms, no difference for visibility as bytes. Beside the next
+// band's contraction, on a stream of its own, it got too few of an SM's registers to keep up and held back the downloads
+// (the 8200-sensor call 1710 us).
+constexpr uint32_t kSunRows = 64, kSunCols = 64, kSunWarpRows = 16;
 __device__ __forceinline__ uint32_t sun_seg_of(const TcGroup& g, uint32_t block) {
   uint32_t lo = 0, hi = g.nSegs - 1;
   while (lo < hi) {
@@ -417,39 +420,33 @@ __device__ __forceinline__ uint32_t sun_seg_of(const TcGroup& g, uint32_t block)
   return lo;
 }
 __global__ void __launch_bounds__(256) k_series_sun(const __grid_constant__ TcGroup g) {
-  __shared__ uint32_t term[kSunCols][kSunRows + 1];
-  __shared__ int32_t jOf[kSunCols];
   const TcSeg& a = g.seg[sun_seg_of(g, blockIdx.x)];
   const uint32_t colBlocks = (a.T + kSunCols - 1) / kSunCols, local = blockIdx.x - a.sunBase;
-  const uint32_t r0 = a.mBase * BM + (local / colBlocks) * kSunRows, t0 = (local % colBlocks) * kSunCols;
-  const uint32_t rowEnd = min(a.nc, (a.mBase + a.mTiles) * BM);
-  if (threadIdx.x < kSunCols) jOf[threadIdx.x] = t0 + threadIdx.x < a.T ? __ldg(a.sunOfCol + t0 + threadIdx.x) : -1;
-  __syncthreads();
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t row = r0 + lane;
-  float nrm[3] = {0.f, 0.f, 0.f};
-  if (row < rowEnd) { nrm[0] = a.N[3 * row]; nrm[1] = a.N[3 * row + 1]; nrm[2] = a.N[3 * row + 2]; }
-  for (uint32_t c = warp; c < kSunCols; c += 8) {
-    const int j = jOf[c];
-    uint32_t u = kNoTerm;
-    if (j >= 0 && row < rowEnd) {
-      const uint32_t d = a.sun0 + uint32_t(j);
-      float at;
-      if (a.bytes) { const uint32_t b = a.bytes[size_t(d) * a.nc + row]; at = b ? float(b) / 255.f : 0.f; }
-      else at = float((a.bits[size_t(d >> 5) * a.nc + row] >> (d & 31)) & 1u);
-      if (at != 0.f) u = __float_as_uint(__fmul_rn(__fmul_rn(fmaxf(dotf_rn(nrm, a.sunVec + 3 * j), 0.f), at), a.sunW[j]));
-    }
-    term[c][lane] = u;
-  }
-  __syncthreads();
-  for (uint32_t r = warp; r < kSunRows; r += 8) {
-    const uint32_t i = r0 + r;
-    if (i >= rowEnd) break;
-    float* Erow = a.E + size_t(i) * a.T;
+  const uint32_t r0 = a.mBase * BM + (local / colBlocks) * kSunRows + (warp >> 1) * kSunWarpRows;
+  const uint32_t t = (local % colBlocks) * kSunCols + (warp & 1) * 32 + lane;
+  const uint32_t rowEnd = min(min(a.nc, (a.mBase + a.mTiles) * BM), r0 + kSunWarpRows);
+  const int j = t < a.T ? __ldg(a.sunOfCol + t) : -1;
+  if (j < 0) return;
+  const float sun[3] = {a.sunVec[3 * j], a.sunVec[3 * j + 1], a.sunVec[3 * j + 2]}, w = a.sunW[j];
+  const uint32_t d = a.sun0 + uint32_t(j);
+  const uint32_t* word = a.bits + size_t(d >> 5) * a.nc;
+  const uint8_t* byte = a.bytes ? a.bytes + size_t(d) * a.nc : nullptr;
+  float* E = a.E + t;
+  for (uint32_t i0 = r0; i0 < rowEnd; i0 += 4) {
+    float at[4], e[4];
 #pragma unroll
-    for (uint32_t h = 0; h < kSunCols / 32; ++h) {
-      const uint32_t c = h * 32 + lane, u = term[c][r];
-      if (u != kNoTerm) Erow[t0 + c] = __fadd_rn(Erow[t0 + c], __uint_as_float(u));
+    for (uint32_t q = 0; q < 4; ++q) {
+      const uint32_t i = min(i0 + q, rowEnd - 1);
+      at[q] = byte ? float(__ldg(byte + i)) / 255.f : float((__ldg(word + i) >> (d & 31)) & 1u);
+      e[q] = E[size_t(i) * a.T];
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+      const uint32_t i = i0 + q;
+      if (i >= rowEnd || at[q] == 0.f) continue;
+      const float n[3] = {__ldg(a.N + 3 * i), __ldg(a.N + 3 * i + 1), __ldg(a.N + 3 * i + 2)};
+      E[size_t(i) * a.T] = __fadd_rn(e[q], __fmul_rn(__fmul_rn(fmaxf(dotf_rn(n, sun), 0.f), at[q]), w));
     }
   }
 }
