@@ -323,8 +323,8 @@ struct Engine {
   size_t i0 = 0, visN = 0;
   Buf dc, contrib;   // contrib: one (bin, contribution) pair per path of a bounce launch
   Buf border;        // a bounce launch's samples in tracing order
-  Buf bq;            // a bounce launch's two queues of paths that go on
-  int gridStep = 0;
+  Buf bq;            // a bounce launch's queue of paths that go on
+  int gridRest = 0;
   Buf slotLog;       // ln tn per slot as a float pair (glass transmission)
   size_t nBins = 0, dcN = 0, dcI0 = 0;
   Buf viewCls, viewDist, rowSin;
@@ -351,7 +351,7 @@ struct Engine {
   int gridBits = 0, gridBytes = 0, gridView = 0;
   int builder = 1;            // 1 device LBVH with treelet restructuring (default), 0 host binned SAH (kgb_set_builder)
   uint32_t nodeLimit = 0;     // kgb_set_limits: the walks see only this many of the BVH's nodes (0: all)
-  uint64_t bounceLimitNs = kBounceLimitNs;   // kgb_set_limits: a bounce step kernel's time limit
+  uint64_t bounceLimitNs = kBounceLimitNs;   // kgb_set_limits: a bounce launch's time limit
   uint64_t seriesWaitNs = 0;                  // kgb_set_limits: the series pipeline's wait limit (0: its default)
   bool withholdFills = false;                 // kgb_set_limits: KGB_LIMIT_WITHHOLD_FILLS
   std::vector<DevMesh*> meshes;               // meshes read to the device, by id (null: freed)
@@ -1241,22 +1241,22 @@ KGB_API int kgb_bounce(kgb_engine* e, size_t i0, size_t nc, uint32_t rayFlags, c
   a.slotLog = static_cast<const float2*>(g.slotLog.p);
   a.dc = static_cast<float*>(g.dc.p); a.status = static_cast<uint32_t*>(g.ctl.p) + 1;
   a.limitNs = g.bounceLimitNs;
-  // paths of a launch: at most 2^23 (their results 64 MiB, the two queues of paths that go on 768 MiB)
+  // paths of a launch: at most 2^23 (their results 64 MiB, the queue of paths that go on 384 MiB)
   const size_t nCap = std::max<size_t>(1, (size_t(1) << 23) / nc);
-  if (!g.gridStep) g.gridStep = g.numSMs * bounce_step_blocks_per_sm();
+  if (!g.gridRest) g.gridRest = g.numSMs * bounce_rest_blocks_per_sm();
   // the reference starts at 2^13 / nc samples (1..64); here also at least ~4 paths per resident thread (a path a thread)
   const size_t fill = (size_t(4) * size_t(g.numSMs) * 2048 + nc - 1) / nc;
   for (size_t done = 0, n = std::max(std::clamp<size_t>((size_t(1) << 13) / nc, 1, 64), fill); done < b->M;) {
     if (b->cancel && b->cancel(b->cancelCtx)) return fail("cancelled");
     n = std::min({n, size_t(b->M) - done, nCap});
-    if (!grow(g.contrib, n * nc * 8) || !grow(g.bq, 2 * n * nc * bounce_state_bytes())) return 0;
+    if (!grow(g.contrib, n * nc * 8) || !grow(g.bq, n * nc * bounce_state_bytes())) return 0;
     a.contrib = static_cast<uint2*>(g.contrib.p);
     a.s0 = uint32_t(done); a.s1 = uint32_t(done + n);
     if (!bounce_order(g, a.s0, a.s1, b->M)) return 0;
     a.order = static_cast<const uint32_t*>(g.border.p);
     if (!reset_ctl(g)) return 0;
     CU(cudaEventRecord(g.ev[0], g.st));
-    launch_bounce(a, static_cast<PathState*>(g.bq.p), static_cast<uint32_t*>(g.ctl.p) + 28, g.gridStep, g.st);
+    launch_bounce(a, static_cast<PathState*>(g.bq.p), static_cast<uint32_t*>(g.ctl.p) + 28, g.gridRest, g.st);
     CU(cudaEventRecord(g.ev[1], g.st));
     uint32_t ctl[32] = {};
     CU(cudaMemcpyAsync(ctl, g.ctl.p, 128, cudaMemcpyDeviceToHost, g.st));

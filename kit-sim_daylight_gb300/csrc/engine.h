@@ -76,7 +76,7 @@ struct ViewArgs {
   uint32_t* status;
 };
 
-// The bounce's step kernels end their remaining paths and fail the call once a step has run this long.
+// k_bounce_rest ends its remaining paths, and the call fails, once it has run this long.
 constexpr uint64_t kBounceLimitNs = 10000000000ull;   // 10 s
 
 struct PathState;   // a path between segments (trace.cu)
@@ -97,11 +97,10 @@ struct BounceArgs {
   uint32_t* status;
   const uint32_t* order;   // [s1 - s0]: the launch's samples in tracing order (sensor-major), or null (sample-major)
   const float2* slotLog;   // [nSlots]: ln tn per slot as a float pair (k_slot_logs)
-  const PathState* qIn;    // the paths a step continues, and their count
-  const uint32_t* qInCount;
-  PathState* qOut;         // the paths that go on after it, appended
-  uint32_t* qOutCount;
-  uint64_t limitNs;        // a step kernel's time limit (kBounceLimitNs unless lowered by kgb_set_limits)
+  PathState* queue;        // the paths that go on after their first segment, their count, and the next one to take
+  uint32_t* qCount;
+  uint32_t* qNext;
+  uint64_t limitNs;        // k_bounce_rest's time limit (kBounceLimitNs unless lowered by kgb_set_limits)
 };
 
 void launch_ray_table(const float* D, uint32_t nDir, void* tab, cudaStream_t st);   // 48 bytes per direction
@@ -123,9 +122,9 @@ int bits_blocks_per_sm();
 void launch_bits(const TraceArgs& a, int resident, cudaStream_t st, bool count = false);
 void launch_bytes(const TraceArgs& a, int resident, cudaStream_t st);
 void launch_view(const ViewArgs& a, int resident, cudaStream_t st);
-void launch_bounce(const BounceArgs& a, PathState* queues, uint32_t* qCount, int stepGrid, cudaStream_t st);
+void launch_bounce(const BounceArgs& a, PathState* queue, uint32_t* qCount, int restGrid, cudaStream_t st);
 size_t bounce_state_bytes();   // one queued path
-int bounce_step_blocks_per_sm();
+int bounce_rest_blocks_per_sm();
 
 // reductions (reduce.cu)
 // w64: a device array of nDir doubles for the weights, or null (the weights staged per block in shared memory: for callers
