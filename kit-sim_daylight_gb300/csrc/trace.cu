@@ -548,14 +548,30 @@ __global__ void __launch_bounds__(128) k_bounce_rest(BounceArgs a) {
     atomicOr(a.status, (overflow & 1u ? kStatusStackOverflow : 0u) | (overflow & 2u ? kStatusVisitLimit : 0u) | (late ? kStatusTimeout : 0u));
 }
 
-// Per sensor, the launch's samples in order: row[bin] = row[bin] + contribution (the reference's float additions).
-__global__ void __launch_bounds__(256) k_bounce_accum(BounceArgs a) {
+// Per sensor, the launch's samples in order: row[bin] = row[bin] + contribution (the reference's float additions). A
+// thread's additions wait on reads of its results and of its rows: it reads eight results, then their bins' rows, at once, and
+// a bin met again among them goes on from the sum it already has (20,011 sensors x 1024 paths: the call 11.5 to 10.9 ms).
+__global__ void __launch_bounds__(64) k_bounce_accum(BounceArgs a) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
+  constexpr uint32_t B = 8;
   float* row = a.dc + i;
-  for (uint32_t q = 0; q < a.s1 - a.s0; ++q) {
-    const uint2 c = a.contrib[size_t(q) * a.n + i];
-    if (c.x != kNoBin) { float* p = row + size_t(c.x) * a.nc; *p = *p + __uint_as_float(c.y); }
+  const uint32_t S = a.s1 - a.s0;
+  for (uint32_t q0 = 0; q0 < S; q0 += B) {
+    uint2 c[B];
+    float v[B];
+#pragma unroll
+    for (uint32_t k = 0; k < B; ++k) c[k] = q0 + k < S ? __ldcs(a.contrib + size_t(q0 + k) * a.n + i) : make_uint2(kNoBin, 0u);
+#pragma unroll
+    for (uint32_t k = 0; k < B; ++k) v[k] = c[k].x != kNoBin ? row[size_t(c[k].x) * a.nc] : 0.f;
+#pragma unroll
+    for (uint32_t k = 0; k < B; ++k) {
+#pragma unroll
+      for (uint32_t j = 0; j < k; ++j) if (c[j].x == c[k].x) v[k] = v[j];
+      v[k] = v[k] + __uint_as_float(c[k].y);
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < B; ++k) if (c[k].x != kNoBin) row[size_t(c[k].x) * a.nc] = v[k];
   }
 }
 
@@ -668,7 +684,7 @@ void launch_bounce(const BounceArgs& args, PathState* queue, uint32_t* qCount, i
   cudaMemsetAsync(qCount, 0, 8, st);
   k_bounce_paths<<<unsigned((paths + 127) / 128), 128, 0, st>>>(a);
   k_bounce_rest<<<restGrid, 128, 0, st>>>(a);
-  k_bounce_accum<<<(a.n + 255) / 256, 256, 0, st>>>(a);
+  k_bounce_accum<<<(a.n + 63) / 64, 64, 0, st>>>(a);
 }
 size_t bounce_state_bytes() { return sizeof(PathState); }
 int bounce_rest_blocks_per_sm() {   // resident blocks of k_bounce_rest per SM (its grid fills the GPU once)
