@@ -1244,8 +1244,9 @@ KGB_API int kgb_bounce(kgb_engine* e, size_t i0, size_t nc, uint32_t rayFlags, c
   // paths of a launch: at most 2^23 (their results 64 MiB, the queue of paths that go on 384 MiB)
   const size_t nCap = std::max<size_t>(1, (size_t(1) << 23) / nc);
   if (!g.gridRest) g.gridRest = g.numSMs * bounce_rest_blocks_per_sm();
-  // the reference starts at 2^13 / nc samples (1..64); here also at least ~4 paths per resident thread (a path a thread)
-  const size_t fill = (size_t(4) * size_t(g.numSMs) * 2048 + nc - 1) / nc;
+  // the reference starts at 2^13 / nc samples (1..64); here also at least ~16 paths per resident thread (a path a thread):
+  // a few ms, in which a launch's last paths count little (20,011 sensors x 1024 paths: 3 launches, 10.6 ms; 5 from 4, 10.9)
+  const size_t fill = (size_t(16) * size_t(g.numSMs) * 2048 + nc - 1) / nc;
   for (size_t done = 0, n = std::max(std::clamp<size_t>((size_t(1) << 13) / nc, 1, 64), fill); done < b->M;) {
     if (b->cancel && b->cancel(b->cancelCtx)) return fail("cancelled");
     n = std::min({n, size_t(b->M) - done, nCap});
