@@ -5,7 +5,7 @@ import pytest
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("nc,M,N", [(1, 1, 1), (1, 1000, 0), (33, 7, 5), (257, 129, 2), (4001, 9, 1), (3000, 65, 3)])
+@pytest.mark.parametrize("nc,M,N", [(1, 1, 1), (1, 1000, 0), (33, 7, 5), (257, 129, 2), (4001, 9, 1), (4001, 16, 1), (3000, 65, 3)])
 def test_rows(engine_lib, oracle, kgb, pkg, nc, M, N):
     s = pkg.workloads.random_city(5, porous=True, glass=True, thin=True)
     slots = [(0.2, 0, 0, 0), (0.3, 0.5, 0, 0), (0.0, 0.64, kgb.tn_from_Tn(0.64), kgb.SLOT_GLASS), (0.25, 0, 0, 0), (0.2, 0, 0, 0),
