@@ -435,12 +435,116 @@ __global__ void __launch_bounds__(32 * kSumWarps) k_sum_warp(S t, uint32_t n, co
   out[i] = odd ? fp64_sum<COS>(t, n, W, i) : __longlong_as_double((long long)os_bits(s));
 }
 
+// The same sum by a block, for few sensors, where a warp a sensor leaves the SMs idle and a word takes it 0.4 us of
+// dependent instructions: a word to each of kBlockWords warps at a time. Each warp rounds its terms on the grid of the
+// sum so far and publishes their total; where no term lies above the grid and the totals keep the sum in its binade, the
+// sum is that much larger. A warp's first halfway term depends on the sum's parity before the warp: its total is given
+// for an even sum, with the difference for an odd one. Otherwise the totals before the first word that leaves the binade
+// are added, that word's warp adds its terms as above, and the words after it are rounded again on the new grid. That is
+// 2.5 us a word that leaves the binade, so it takes sums long enough that most words do not, and no more sensors than
+// three or so an SM (a warp a sensor / 4 / 8 / 16 / 32 warps, us a call with the cosine): 16 sensors x 4746 directions
+// 82 / 65 / 60 / 60 / 63, 300 x 5610 87 / 73 / 69 / 73 / 107, 600 x 5610 89 / 83 / 84 / 109 / 174, 1000 x 5610
+// 97 / 104 / 119 / 151 / 262; 100 x 9066 bytes 124 / 90 / 77 / 76 / 83; 100 x 1290 49 / 50 / 48 / 49 / 55.
+constexpr uint32_t kBlockWords = 8;
+struct WordTotal {
+  uint64_t even;    // the total, given an even sum before it
+  int32_t odd;      // what an odd sum before it adds: 0, 1 or -1
+  uint32_t flags;   // 1: the sum's parity after it (after its last halfway term, if any); 2: halfway terms; 4: adds alone
+};
+__device__ __forceinline__ WordTotal word_total(const OrderedSum& s, uint64_t p, int32_t e, uint32_t lane) {
+  const int32_t sh = s.g - e;
+  const uint32_t by = uint32_t(sh) < 63u ? uint32_t(sh) : 63u;
+  const uint64_t rem = (p << (63u - by)) << 1, half = 1ull << 63;
+  uint64_t r = (p >> by) + (rem > half ? 1u : 0u);
+  WordTotal t{0, 0, 0};
+  t.flags = __any_sync(~0u, p != 0 && (sh < 0 || !s.a)) ? 4u : 0u;
+  const uint32_t ties = __ballot_sync(~0u, rem == half), odd = __ballot_sync(~0u, uint32_t(r) & 1u);
+  uint32_t after = odd;
+  if (ties) {
+    const uint32_t below = (1u << lane) - 1u, last = ties & below;
+    const uint32_t since = last ? below & (~1u << (31 - __clz(last))) : below;
+    const uint32_t bump = (__popc(odd & since) & 1u) ^ (uint32_t(r) & 1u);
+    if (ties >> lane & 1u) r += bump;
+    t.odd = __shfl_sync(~0u, bump, __ffs(ties) - 1) ? -1 : 1;
+    after = odd & (~1u << (31 - __clz(ties)));
+    t.flags |= 2u;
+  }
+  t.flags |= __popc(after) & 1u;
+  t.even = __reduce_add_sync(~0u, uint32_t(r) & 0xffffffu) + (uint64_t(__reduce_add_sync(~0u, uint32_t(r >> 24))) << 24);
+  return t;
+}
+template <bool COS, class S>
+__global__ void __launch_bounds__(32 * kBlockWords) k_sum_block(S t, uint32_t n, const uint2* __restrict__ W, double* __restrict__ out) {
+  __shared__ WordTotal tot[2][kBlockWords];
+  __shared__ OrderedSum left;
+  const uint32_t i = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+  const F3 v = t.sensor(i);
+  OrderedSum s;
+  bool odd = false;
+  typename S::Raw raw;
+  F3 dir{};
+  uint2 w;
+  const auto read = [&](uint32_t d0) {
+    const uint32_t d = min(d0 + threadIdx.x, n - 1);
+    raw = t.raw(d, i);
+    if (COS) dir = ld3(t.D + 3 * d);
+    w = __ldg(W + d);
+  };
+  read(0);
+  uint32_t turn = 0;
+  for (uint32_t d0 = 0; d0 < n; d0 += 32 * kBlockWords) {
+    uint64_t p;
+    int32_t e;
+    const uint32_t d = d0 + threadIdx.x;
+    term(d < n ? t.factor(raw, d, cosine<COS>(v, dir)) : 0.f, w, p, e, odd);
+    if (d0 + 32 * kBlockWords < n) read(d0 + 32 * kBlockWords);   // under way while these are added
+    for (uint32_t from = 0; from < kBlockWords;) {   // the words before it are added
+      const WordTotal mine = word_total(s, p, e, lane);
+      WordTotal* all = tot[turn++ & 1u];
+      if (!lane) all[warp] = warp < from ? WordTotal{0, 0, 0} : mine;
+      __syncthreads();
+      const WordTotal x = lane < kBlockWords ? all[lane] : WordTotal{0, 0, 0};
+      uint64_t r = x.even;
+      const uint32_t ties = __ballot_sync(~0u, x.flags & 2u);
+      if (ties) {
+        const uint32_t parity = __ballot_sync(~0u, x.flags & 1u), below = (1u << lane) - 1u, last = ties & below;
+        const uint32_t since = last ? below & (~0u << (31 - __clz(last))) : below;
+        if ((__popc(parity & since) & 1u) ^ (last ? 0u : uint32_t(s.a) & 1u)) r += int64_t(x.odd);
+      }
+      const uint32_t alone = __ballot_sync(~0u, x.flags & 4u);
+      const uint64_t a = s.a + __reduce_add_sync(~0u, uint32_t(r) & 0x7ffffffu) + (uint64_t(__reduce_add_sync(~0u, uint32_t(r >> 27))) << 27);
+      if (!alone && !(a >> 53)) { s.a = a; break; }
+      uint64_t upTo = r;   // the totals up to and with the lane's word
+#pragma unroll
+      for (int o = 1; o < int(kBlockWords); o <<= 1) {
+        const uint64_t y = uint64_t(__shfl_up_sync(~0u, uint32_t(upTo), o)) | uint64_t(__shfl_up_sync(~0u, uint32_t(upTo >> 32), o)) << 32;
+        if (lane >= uint32_t(o)) upTo += y;
+      }
+      const uint32_t at = __ffs(alone | __ballot_sync(~0u, (s.a + upTo) >> 53)) - 1;
+      const uint64_t less = upTo - r;
+      s.a += uint64_t(__shfl_sync(~0u, uint32_t(less), at)) | uint64_t(__shfl_sync(~0u, uint32_t(less >> 32), at)) << 32;
+      if (warp == at) {
+        add_32(s, p, e, lane);
+        if (!lane) left = s;
+      }
+      __syncthreads();
+      s = left;
+      from = at + 1;
+    }
+  }
+  if (__syncthreads_or(odd)) {
+    if (!threadIdx.x) out[i] = fp64_sum<COS>(t, n, W, i);
+  } else if (!threadIdx.x) out[i] = __longlong_as_double((long long)os_bits(s));
+}
+
 static uint32_t blocks_of(uint32_t n) { return (n + kReduceBlock - 1) / kReduceBlock; }
+constexpr uint32_t kBlockSensors = 450, kBlockDirs = 2048;
 template <bool COS, class S>
 static void launch_sum_warp(const S& t, uint32_t n, const float* W, double* w64, double* out, cudaStream_t st) {
   uint2* parts = reinterpret_cast<uint2*>(w64);
   k_weight_parts<<<(n + 255) / 256, 256, 0, st>>>(W, n, parts);
-  k_sum_warp<COS><<<(t.nc + kSumWarps - 1) / kSumWarps, 32 * kSumWarps, 0, st>>>(t, n, parts, out);
+  if (t.nc <= kBlockSensors && n >= kBlockDirs) k_sum_block<COS><<<t.nc, 32 * kBlockWords, 0, st>>>(t, n, parts, out);
+  else k_sum_warp<COS><<<(t.nc + kSumWarps - 1) / kSumWarps, 32 * kSumWarps, 0, st>>>(t, n, parts, out);
 }
 // Which form is faster (152 SMs): the thread form waits some 70 ns a direction for its fma and its reads (bits without
 // the cosine; 110 ns with it, 140 and 180 ns bytes), whatever the sensors, until they fill the SMs; the warp form costs
