@@ -816,8 +816,8 @@ static int trace_impl(Engine& g, size_t i0, size_t nc, uint32_t rayFlags, uint64
     a.first = uint32_t(i0 + done); a.n = uint32_t(n); a.out0 = uint32_t(done); a.p0 = uint32_t(done);
     a.frontiers = nullptr;
     if (g.nDir >= kFrontierDirs && n * g.nDir >= kFrontierRays) {
-      if (!grow(g.frontiers, (n + 31) / 32 * frontier_bytes())) return 0;
-      a.frontiers = static_cast<FrontierRec*>(g.frontiers.p);
+      if (grow(g.frontiers, (n + 31) / 32 * frontier_bytes())) a.frontiers = static_cast<FrontierRec*>(g.frontiers.p);
+      else cudaGetLastError();   // no room for the records: the walks start at the root
     }
     if (!reset_ctl(g)) return 0;
     CU(cudaEventRecord(g.ev[0], g.st));

@@ -3,11 +3,11 @@
 //  k_bytes  transmittance bytes (replaces __raygen__bytes + __anyhit__tr, trace_dev.cu:115-165)
 //  k_view   class + distance of the closest hit per view cell (replaces __raygen__view, trace_dev.cu:177-232)
 //  k_bounce_paths, k_bounce_rest, k_bounce_accum, k_bounce_accum_few
-//           reflected-light paths binned by sky patch (replaces __raygen__bounce, trace_dev.cu:260-311), : first
+//           reflected-light paths binned by sky patch (replaces __raygen__bounce, trace_dev.cu:260-311): first
 //           segments, then the paths that go on from a queue, to their ends
 // The visibility kernels are persistent: each warp takes tasks of 32 consecutive sensors x up to 32 directions from a
-// global counter, so a warp traces one direction for 32 neighbouring sensors at a time (coherent rays). k_bits
-// and k_bytes take a call's sensors in the engine's tracing order (grouped by the orientation of their normals:
+// global counter, so a warp traces one direction for 32 neighbouring sensors at a time (coherent rays; k_view: two cells
+// for 16). k_bits and k_bytes take a call's sensors in the engine's tracing order (grouped by the orientation of their normals:
 // TraceArgs::order), so that a warp's sensors face the same way more often; each result goes to its sensor's column.
 #include "engine.h"
 #include "rt.cuh"
