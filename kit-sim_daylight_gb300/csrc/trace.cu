@@ -39,7 +39,8 @@ __device__ __forceinline__ uint32_t next_task(uint32_t* counter) {
 // ---------------------------------------------------------------------------------------------------- bits
 // Direction d of a sensor is visible when n.d > 0 and every hit from tmin 1e-5 on is an own-plane hit, at most 3.
 // A task is 32 sensors x PER directions of a word (32, 16 or 8: task_directions; a template, since the whole word's form
-// keeps 80 registers without spills and the general one did not: 2 % of the urban trace). FRONT: the walks start from the
+// keeps 80 registers without spills and the general one did not: 2 % of the urban trace); the parts of the last word past
+// the last direction are no tasks (199,000 sensors x 14 directions 208 to 201 us). FRONT: the walks start from the
 // 32 sensors' frontier (a.frontiers, by position in the launch), which k_frontiers made.
 // COUNT: the instrumented variant (same results) that adds up nodes visited, triangles tested and rays traced.
 template <bool COUNT, uint32_t PER, bool FRONT>
@@ -48,7 +49,7 @@ __global__ void __launch_bounds__(256) k_bits(TraceArgs a) {
   const Scene s{a.nodes, a.tris, a.nNodes};
   const bool cull = (a.rayFlags & KGB_RAY_CULL_BACK_FACING) != 0;
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t cols = a.nWords * (32 / PER), nTasks = (a.n + 31) / 32 * cols;
+  const uint32_t cols = (a.nDir + PER - 1) / PER, nTasks = (a.n + 31) / 32 * cols;
   uint32_t overflow = 0;
   Count ctr;
   uint32_t rays = 0;
@@ -77,8 +78,13 @@ __global__ void __launch_bounds__(256) k_bits(TraceArgs a) {
     uint32_t* out = a.bits + size_t(e0 / 32) * a.stride + col;
     const uint32_t at = e0 % 32;
     if (PER == 32) *out = word;
-    else if (PER == 16) reinterpret_cast<uint16_t*>(out)[at / 16] = uint16_t(word >> at);
-    else reinterpret_cast<uint8_t*>(out)[at / 8] = uint8_t(word >> at);
+    else if (PER == 16) {
+      reinterpret_cast<uint16_t*>(out)[at / 16] = uint16_t(word >> at);
+      if (!at && e0 + 16 >= a.nDir) reinterpret_cast<uint16_t*>(out)[1] = 0;   // no task for the word's second half
+    } else {
+      reinterpret_cast<uint8_t*>(out)[at / 8] = uint8_t(word >> at);
+      if (e0 + 8 >= a.nDir) for (uint32_t k = at / 8 + 1; k < 4; ++k) reinterpret_cast<uint8_t*>(out)[k] = 0;   // no tasks for these
+    }
   }
   if (overflow) atomicOr(a.status, (overflow & 1u ? kStatusStackOverflow : 0u) | (overflow & 2u ? kStatusVisitLimit : 0u));
   if (COUNT) {
@@ -675,7 +681,7 @@ void launch_bits(const TraceArgs& a, int resident, cudaStream_t st, bool count) 
   const size_t blocks = (size_t(a.n) + 31) / 32, words = blocks * a.nWords, warps = size_t(resident) * 8;
   if (!count && 4 * words < warps) { k_bits_few<<<unsigned(words), 32 * kFewWarps, 0, st>>>(a); return; }
   const uint32_t per = count ? 32u : task_directions(blocks, size_t(a.nWords) * 32, warps, 8);
-  const int grid = task_grid(words * (32 / per), resident);
+  const int grid = task_grid(blocks * ((a.nDir + per - 1) / per), resident);
   const bool front = a.frontiers != nullptr;
   if (front) launch_frontiers(a, blocks, st);
   if (count) front ? k_bits<true, 32, true><<<grid, 256, 0, st>>>(a) : k_bits<true, 32, false><<<grid, 256, 0, st>>>(a);

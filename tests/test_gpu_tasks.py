@@ -30,3 +30,28 @@ def test_bits_bytes_views(engine_lib, oracle, kgb, pkg, nc, n_dir):
     finally:
         e.close()
         o.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nc,n_dir", [(6000, 301), (6251, 1217), (6251, 4121), (6251, 19075)])
+def test_bits_past_the_directions(engine_lib, oracle, kgb, pkg, nc, n_dir):
+    """The last word's bits past the last direction are zero where tasks of 8 or 16 directions end before it, whatever the
+    buffer held (a byte trace, before)."""
+    s = pkg.workloads.random_city(3)
+    D = pkg.workloads.hemisphere_dirs(n_dir, 1, nc)[:n_dir]
+    check = np.concatenate([np.arange(16), np.arange(nc - 16, nc)])   # the oracle traces these
+    e, o = kgb.Engine(engine_lib), kgb.Engine(oracle)
+    try:
+        for x, pick in ((e, np.arange(nc)), (o, check)):
+            x.build(s["v"], s["tri"])
+            x.set_scene(s["P"][pick], s["N"][pick], D)
+        e.trace(0, nc, 4)
+        e.trace(0, nc, 5)
+        o.trace(0, len(check), 5)
+        bits = e.download_bits(nc)
+        assert np.array_equal(bits[:, check], o.download_bits(len(check)))
+        if n_dir % 32:
+            assert not np.any(bits[-1] >> np.uint32(n_dir % 32))
+    finally:
+        e.close()
+        o.close()
