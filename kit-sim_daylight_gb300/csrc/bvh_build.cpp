@@ -3,9 +3,8 @@
 // inner child until it has 8) with float child boxes, stored as the 208-byte node / 48-byte triangle records rt.cuh
 // reads.
 //
-// Conservative by construction: every triangle box is expanded by prim_eps (engine.h; the bound is at kWiden in rt.cuh)
-// before anything is built, so a box test never drops a triangle the watertight test would report; the traversal then
-// equals the brute-force hit set on any input.
+// Every triangle box is expanded by prim_eps (engine.h; the bound, and the hits it leaves out, are at kWiden in rt.cuh)
+// before anything is built, so that a box test drops no triangle the watertight test would report.
 #include "engine.h"
 
 #include <algorithm>
@@ -105,7 +104,8 @@ void build_bvh8(const float* v, size_t nv, const uint32_t* tri, size_t nt, const
       L = std::max({L, std::fabs(e1[a]), std::fabs(e2[a]), std::fabs(p[2][a] - p[1][a])});
     }
     const float nx = e1[1] * e2[2] - e1[2] * e2[1], ny = e1[2] * e2[0] - e1[0] * e2[2], nz = e1[0] * e2[1] - e1[1] * e2[0];
-    const float eps = prim_eps(L, std::sqrt(nx * nx + ny * ny + nz * nz), M);
+    const auto flat = [&](int a) { return p[0][a] == p[1][a] && p[0][a] == p[2][a]; };
+    const float eps = prim_eps(flat(0) || flat(1) || flat(2), L, std::sqrt(nx * nx + ny * ny + nz * nz), M);
     for (int a = 0; a < 3; ++a) {
       const float lo = std::min({p[0][a], p[1][a], p[2][a]}), hi = std::max({p[0][a], p[1][a], p[2][a]});
       B.tb[k].lo[a] = lo - eps; B.tb[k].hi[a] = hi + eps;

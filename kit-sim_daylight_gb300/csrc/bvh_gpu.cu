@@ -18,8 +18,8 @@
 //      sorted order), and a prefix sum over the level gives each node its block of inner children and of triangle
 //      records, so the layout is deterministic
 //   7. each node's child boxes written as floats (the expanded boxes of step 2, merged), empty slots +inf / -inf
-// Conservative exactly as the host builder: any conservative BVH gives the traversal the brute-force hit set, so the
-// results do not depend on which builder made the scene.
+// Conservative exactly as the host builder (the bound, and the grazing hits it leaves out: kWiden, rt.cuh), so the results
+// do not depend on which builder made the scene.
 #include "engine.h"
 
 #include <cub/device/device_radix_sort.cuh>
@@ -61,7 +61,9 @@ __global__ void k_prims(const float* v, const uint32_t* tri, uint32_t nt, float 
     const float L = fmaxf(fmaxf(fmaxf(fabsf(ax), fabsf(ay)), fmaxf(fabsf(az), fabsf(bx))),
                           fmaxf(fmaxf(fabsf(by), fabsf(bz)), fmaxf(fabsf(p2[0] - p1[0]), fmaxf(fabsf(p2[1] - p1[1]), fabsf(p2[2] - p1[2])))));
     const float nx = ay * bz - az * by, ny = az * bx - ax * bz, nz = ax * by - ay * bx;
-    const float eps = prim_eps(L, sqrtf(nx * nx + ny * ny + nz * nz), M);
+    bool flat = false;
+    for (int a = 0; a < 3; ++a) flat = flat || (p0[a] == p1[a] && p0[a] == p2[a]);
+    const float eps = prim_eps(flat, L, sqrtf(nx * nx + ny * ny + nz * nz), M);
     for (int a = 0; a < 3; ++a) {
       const float x0 = p0[a], x1 = p1[a], x2 = p2[a];
       const float mn = fminf(x0, fminf(x1, x2)), mx = fmaxf(x0, fmaxf(x1, x2));

@@ -278,17 +278,17 @@ std::string thin_solids(const double* points, size_t nPoints, const int32_t* cou
 const char* sky_ladybug(int mf, const double* steps, size_t T, double lat, double lon, double tz, double grefl, double durationHours,
                         double* lb, float* acc, float* S, float* g, cudaStream_t st);
 
-// By how much a triangle's box is expanded on each side (why: kWiden, rt.cuh), given its extent L along the axes, area2
-// (twice its area) and M, the scene's largest coordinate (at least 1): 2^-21 M, and 2^-19 L, times L^2 / area2 for a
-// sliver, whose hit distance is that much less certain (a well-shaped triangle's ratio is 1 to 2); together at most
-// 2^-16 M, which a triangle without area gets too.
+// By how much a triangle's box is expanded on each side (why: kWiden, rt.cuh), given M, the scene's largest coordinate (at
+// least 1): 2^-16 M, or less for a triangle perpendicular to an axis (flat: its vertices have one coordinate in common):
+// 2^-21 M, and 2^-19 L, times L^2 / area2 for a sliver, whose hit distance is that much less certain, with its extent L
+// along the axes and area2, twice its area (a well-shaped triangle's ratio is 1 to 2).
 #if defined(__CUDACC__)
 __host__ __device__
 #endif
-inline float prim_eps(float L, float area2, float M) {
+inline float prim_eps(bool flat, float L, float area2, float M) {
   const float most = M * (1.f / 65536.f), sq = L * L;
   const float e = M * (1.f / 2097152.f) + (1.f / 524288.f) * L * (area2 < sq ? sq / area2 : 1.f);
-  return e < most ? e : most;   // also where e is not a number
+  return flat && e < most && area2 <= 3.40282347e38f ? e : most;   // most also where e is not a number, or the area's square overflows
 }
 
 // host BVH builder (bvh_build.cpp): binned-SAH binary BVH, collapsed to the 8-wide float-plane layout of rt.cuh

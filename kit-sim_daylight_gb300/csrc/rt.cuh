@@ -284,20 +284,29 @@ __device__ __forceinline__ unsigned long long pku(uint32_t a, uint32_t b) {
 }
 
 // What the box test owes a hit that the triangle test computes, with u = 2^-24 (a float's half ulp), t the hit's
-// distance, L the triangle's extent, M the scene's largest coordinate:
-//  - the watertight test signs its edge functions exactly for vertices slightly off where they are relative to the ray:
+// distance, L the triangle's extent, K = L^2 / (2 area), M the scene's largest coordinate:
+//  - the triangle test signs its edge functions exactly for vertices slightly off where they are relative to the ray:
 //    subtracting the origin, shearing and rounding the result move them by at most 4 u t |d_a| + 6 u L along axis a
-//    (Sx times the depth is t |d_a| up to L, and so is the vertex's offset). So the ray passes within that of the triangle,
-//    and 4 u t |d_a| is 4 u of the axis's slab distance;
+//    (Sx times the depth is t |d_a| up to L, and so is the vertex's offset). So the ray's line passes within that of the
+//    triangle, and 4 u t |d_a| is 4 u of the axis's slab distance;
+//  - t is the depth of the vertices weighted by the edge functions. A weight is off by some u L^2 over the triangle's area
+//    as seen along the ray, and t by as much of L: up to some u L K / s, s the sine of the ray against the triangle's plane;
+//  - not so for a triangle perpendicular to an axis: its sheared coordinates across that axis are its depths times the
+//    shear (plus its one distance from the origin), so their errors shrink with s as that area does. The weights move t by
+//    at most 12 u L K, the other roundings by 14 u L and a few u of itself, at any incidence;
 //  - a slab distance fma(plane, 1 / d, -o / d) is off by 3 u of itself and, for a coordinate |o_a| up to 6 M, by 7 u M in
-//    distance (the products' rounding and the planes'); past 6 M that too is a small part of the slab distance;
-//  - the computed t is off by about 8 u of itself and by a few u L, times L^2 / area for a sliver.
+//    distance (the products' rounding and the planes'); past 6 M that too is a small part of the slab distance.
 // The exit distance is widened by kWiden, 1 + 32 u, which covers the parts relative to t on both sides of the interval;
-// the triangles' boxes are expanded by prim_eps (8 u M and 32 u L L^2 / area), which covers the others.
-// Every box used to be expanded by 256 u M: 6 mm on a 400 m block, more than the 0.1 to 4 mm by which offset_ray lifts
-// a sensor off its face, so every ray began inside the boxes of its own wall and walked down to its triangles. With the
-// walls' boxes behind the sensors the urban block's rays visit about 6.9 nodes instead of 8.2 and test 0.9 triangles instead
-// of 1.9 (trace 57.5 to 43.3 ms); rotated walls' boxes hold their sensors either way.
+// the triangles' boxes are expanded by prim_eps, which covers the others: 8 u M + 32 u L K for triangles perpendicular to
+// an axis, 256 u M for the others. That leaves out, of the others, hits of s < L K / 8 M at worst whose t is off by more: the
+// ray starts within some 30 u L K of the triangle's plane, past its edge, and leaves it nearly along the plane. A walk may
+// miss such a hit, and then that of another tree may not (three of 8 million rays made for it).
+// With 256 u M for every triangle, 6 mm on a 400 m block, more than the 0.1 to 4 mm by which offset_ray lifts a sensor off
+// its face, every ray began inside the boxes of its own wall and walked down to its triangles. With the walls' boxes behind
+// the sensors the urban block's rays visit about 6.9 nodes instead of 8.2 and test 0.9 triangles instead of 1.9 (trace 57.5
+// to 43.3 ms); the boxes of walls turned against the axes hold their sensors either way. (The smaller expansion only along
+// the axis that the triangle is perpendicular to: 7 % slower on the block; for every triangle: the turned ones lose grazing
+// hits that 256 u M keeps, 220 of the 8 million rays, for 0.5 to 2 % of the views' time.)
 constexpr float kWiden = 1.0000019073486328125f;   // 1 + 2^-19
 
 // Child boxes of the node at p against the ray in [tmin, tmax] (tmin >= 0): returns the mask of hit children (bit k),
