@@ -599,15 +599,18 @@ __device__ __forceinline__ uint32_t order_bits(float f) {   // floats as unsigne
 __device__ __forceinline__ float from_order_bits(uint32_t u) { return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u); }
 
 struct Bounds { F3 lo, hi; };   // of a warp's ray origins
+// An origin that is not finite is left out: its rays hit nothing wherever they walk (hit_tri's t is not a number), and the
+// bounds of the others stay finite, without which shaft would drop entries that their rays enter.
 __device__ __forceinline__ Bounds origin_bounds(F3 o, bool valid) {
   Bounds b;
-  const uint32_t none = order_bits(INFINITY);
+  valid = valid && fabsf(o.x) <= FLT_MAX && fabsf(o.y) <= FLT_MAX && fabsf(o.z) <= FLT_MAX;
+  const uint32_t none = order_bits(INFINITY), no = order_bits(-INFINITY);
   b.lo.x = from_order_bits(__reduce_min_sync(~0u, valid ? order_bits(o.x) : none));
   b.lo.y = from_order_bits(__reduce_min_sync(~0u, valid ? order_bits(o.y) : none));
   b.lo.z = from_order_bits(__reduce_min_sync(~0u, valid ? order_bits(o.z) : none));
-  b.hi.x = from_order_bits(__reduce_max_sync(~0u, valid ? order_bits(o.x) : 0u));
-  b.hi.y = from_order_bits(__reduce_max_sync(~0u, valid ? order_bits(o.y) : 0u));
-  b.hi.z = from_order_bits(__reduce_max_sync(~0u, valid ? order_bits(o.z) : 0u));
+  b.hi.x = from_order_bits(__reduce_max_sync(~0u, valid ? order_bits(o.x) : no));
+  b.hi.y = from_order_bits(__reduce_max_sync(~0u, valid ? order_bits(o.y) : no));
+  b.hi.z = from_order_bits(__reduce_max_sync(~0u, valid ? order_bits(o.z) : no));
   return b;
 }
 
@@ -682,7 +685,7 @@ __device__ __forceinline__ void store_frontier(FrontierRec* rec, const Frontier&
 }
 
 // The entries that some ray from within the bounds in r's direction may enter (all the warp's rays have it), as a mask:
-// each ray's own test passes on a subset, rounding included, since every operation is monotonic.
+// each ray's own test passes on a subset, rounding included, since every operation is monotonic (from finite origins).
 struct Mask64 { uint32_t lo, hi; };
 __device__ __forceinline__ Mask64 shaft(const Frontier& f, uint32_t n, const Bounds& b, const Ray& r, uint32_t lane) {
   // the near plane (lo when the direction is positive) against the origin farthest along, the far one against the first
