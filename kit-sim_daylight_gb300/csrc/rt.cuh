@@ -615,12 +615,13 @@ __device__ __forceinline__ Bounds origin_bounds(F3 o, bool valid) {
 }
 
 // The frontier of a warp's rays: from the root, the largest node that holds some of the origins' bounds and is larger
-// than them is opened, until none is or the entries are used up. Returns the entries. Every lane calls it.
+// than them is opened, until none is or the entries are used up: at most kEntries nodes, so that it ends in a damaged tree
+// too (the entries hold every triangle after each). Returns the entries. Every lane calls it.
 __device__ __forceinline__ uint32_t build_frontier(const Scene& s, const Bounds& b, Frontier& f, uint32_t lane) {
   if (!s.nNodes) return 0;
   const float size = fmaxf(fmaxf(b.hi.x - b.lo.x, b.hi.y - b.lo.y), b.hi.z - b.lo.z);
   uint32_t n = 1, node = 0, at = 0;   // the entry that is opened holds `node`
-  for (;;) {
+  for (int opened = 0;;) {
     const uint4* np = reinterpret_cast<const uint4*>(s.nodes + node);
     const uint4 hd = __ldg(np);
     const uint32_t k = lane & 7u, imask = hd.x >> 24, meta = byte_of(k < 4 ? hd.z : hd.w, k & 3u) & 0x7fu;
@@ -637,9 +638,11 @@ __device__ __forceinline__ uint32_t build_frontier(const Scene& s, const Bounds&
       f.open[e] = inner && child < s.nNodes && ext > size && x.x <= b.hi.x && x.y >= b.lo.x && y.x <= b.hi.y && y.y >= b.lo.y && z.x <= b.hi.z &&
                   z.y >= b.lo.z ? ext : 0.f;
     }
-    n += __popc(in) - 1;
+    if (in) n += __popc(in) - 1;
+    else if (!opened) return 0;                 // a root without children
+    else if (lane == 0) f.open[at] = 0.f;       // such a node stays an entry
     __syncwarp();
-    if (n + 7 > kEntries) break;
+    if (n + 7 > kEntries || ++opened == kEntries) break;
     const uint32_t x = lane < n ? __float_as_uint(f.open[lane]) : 0u, y = lane + 32 < n ? __float_as_uint(f.open[lane + 32]) : 0u;
     const uint32_t top = __reduce_max_sync(~0u, max(x, y));
     if (!top) break;
