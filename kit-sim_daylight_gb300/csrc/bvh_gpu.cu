@@ -592,7 +592,7 @@ struct DevBuf {
   ~DevBuf() { if (p) cudaFree(p); }
   template <class T> T* as() { return static_cast<T*>(p); }
 };
-#define KGB_TRY(x) do { const cudaError_t e_ = (x); if (e_ != cudaSuccess) return std::string(#x ": ") + cudaGetErrorString(e_); } while (0)
+#define KGB_TRY(x) do { const cudaError_t e_ = (x); if (e_ != cudaSuccess) { cudaGetLastError(); return std::string(#x ": ") + cudaGetErrorString(e_); } } while (0)   // the error is reported here, not by the next call's check
 
 }  // namespace
 

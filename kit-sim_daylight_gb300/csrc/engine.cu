@@ -39,7 +39,10 @@ int fail(const std::string& m) { g_err = m; return 0; }
 #define CU(call)                                                                          \
   do {                                                                                    \
     cudaError_t e_ = (call);                                                              \
-    if (e_ != cudaSuccess) return fail(std::string(#call) + ": " + cudaGetErrorString(e_)); \
+    if (e_ != cudaSuccess) {                                                              \
+      cudaGetLastError(); /* reported here, not by the next call's launch check */        \
+      return fail(std::string(#call) + ": " + cudaGetErrorString(e_));                    \
+    }                                                                                     \
   } while (0)
 
 struct Buf {   // device buffer, grown as needed (contents not kept)
@@ -816,8 +819,7 @@ static int trace_impl(Engine& g, size_t i0, size_t nc, uint32_t rayFlags, uint64
     a.first = uint32_t(i0 + done); a.n = uint32_t(n); a.out0 = uint32_t(done); a.p0 = uint32_t(done);
     a.frontiers = nullptr;
     if (g.nDir >= kFrontierDirs && n * g.nDir >= kFrontierRays) {
-      if (grow(g.frontiers, (n + 31) / 32 * frontier_bytes())) a.frontiers = static_cast<FrontierRec*>(g.frontiers.p);
-      else cudaGetLastError();   // no room for the records: the walks start at the root
+      if (grow(g.frontiers, (n + 31) / 32 * frontier_bytes())) a.frontiers = static_cast<FrontierRec*>(g.frontiers.p);   // else no room: from the root
     }
     if (!reset_ctl(g)) return 0;
     CU(cudaEventRecord(g.ev[0], g.st));
