@@ -720,14 +720,14 @@ KGB_API uint64_t kgb_free_bytes(void) {
 // every sensor do not depend on the order: any partition of the sensors into six runs, each in index order, traces the
 // same rays, so the order is rebuilt only when the classes of the sensors just uploaded differ from those it was built
 // from (a kernel compares them on the device; a caller that sends the same sensors every step pays for that kernel).
-static bool sensor_order(Engine& g, size_t nSensors) {
+// had: an order was there, and its classes. g.ordered is set once the order is the sensors': an error leaves none.
+static bool sensor_order(Engine& g, size_t nSensors, bool had) {
+  g.ordered = false;
   if (nSensors < kOrderSensors || nSensors * g.nDir < kOrderRays) {   // none: the traces take them as they come
     g.orderHost.clear();
-    g.ordered = false;
     return true;
   }
-  const bool fresh = !g.ordered || g.orderHost.size() != nSensors || !g.order.p;
-  g.ordered = true;
+  const bool fresh = !had || g.orderHost.size() != nSensors || !g.order.p;
   if (!grow(g.cls, nSensors) || !grow(g.clsFlags, 7 * 4)) return false;
   if (fresh) CU(cudaMemsetAsync(g.cls.p, 0xff, nSensors, g.st));   // no class yet: every sensor differs
   CU(cudaMemsetAsync(g.clsFlags.p, 0, 7 * 4, g.st));
@@ -737,12 +737,13 @@ static bool sensor_order(Engine& g, size_t nSensors) {
   CU(cudaMemcpyAsync(g.host + 1, g.clsFlags.p, 7 * 4, cudaMemcpyDeviceToHost, g.st));
   CU(cudaStreamSynchronize(g.st));
   const uint32_t* f = g.host + 1;
-  if (!f[0] && !fresh) return true;
-  std::vector<uint8_t> cls(nSensors);
-  if (nSensors) {
-    CU(cudaMemcpyAsync(cls.data(), g.cls.p, nSensors, cudaMemcpyDeviceToHost, g.st));
-    CU(cudaStreamSynchronize(g.st));
+  if (!f[0] && !fresh) {
+    g.ordered = true;
+    return true;
   }
+  std::vector<uint8_t> cls(nSensors);
+  CU(cudaMemcpyAsync(cls.data(), g.cls.p, nSensors, cudaMemcpyDeviceToHost, g.st));
+  CU(cudaStreamSynchronize(g.st));
   g.classStart[0] = 0;
   for (int c = 0; c < 6; ++c) g.classStart[c + 1] = g.classStart[c] + f[1 + c];
   if (g.classStart[6] != nSensors) return fail("gpu_set_scene: the sensors' classes do not add up");
@@ -750,18 +751,22 @@ static bool sensor_order(Engine& g, size_t nSensors) {
   for (int c = 0; c < 6; ++c) at[c] = g.classStart[c];
   g.orderHost.resize(nSensors);
   for (size_t i = 0; i < nSensors; ++i) g.orderHost[at[cls[i]]++] = uint32_t(i);
-  return upload(g.order, g.orderHost.data(), nSensors * 4, g.st);
+  g.ordered = upload(g.order, g.orderHost.data(), nSensors * 4, g.st);
+  return g.ordered;
 }
 
 KGB_API int kgb_set_scene(kgb_engine* e, const float* P, const float* N, size_t nSensors, const float* D, size_t nDir) {
   Engine& g = *E(e);
   if (nSensors > 0xffffffffull) return fail("gpu_set_scene: more sensors than 32-bit indices hold");
-  g.nSensors = nSensors; g.nDir = nDir; g.nWords = (nDir + 31) / 32;
+  const bool had = g.ordered;
+  g.ordered = false;
+  g.nSensors = g.nDir = g.nWords = 0;   // none until all are there: an error leaves nothing to trace
   if (!upload(g.P, P, nSensors * 12, g.st) || !upload(g.N, N, nSensors * 12, g.st) || !upload(g.D, D, nDir * 12, g.st) ||
       !grow(g.rayTab, nDir * 48)) return 0;
+  g.nSensors = nSensors; g.nDir = nDir; g.nWords = (nDir + 31) / 32;
   launch_ray_table(static_cast<const float*>(g.D.p), uint32_t(nDir), g.rayTab.p, g.st);
   CU(cudaGetLastError());
-  if (!sensor_order(g, nSensors)) return 0;
+  if (!sensor_order(g, nSensors, had)) return 0;
   CU(cudaStreamSynchronize(g.st));
   return 1;
 }

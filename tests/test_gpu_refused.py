@@ -1,5 +1,6 @@
-"""A kgb_set_scene that the device has no room for (here: a direction count beyond any memory) costs the next call
-nothing: the same sensors set again are traced as by an engine that never failed."""
+"""A kgb_set_scene that the device has no room for (here: a direction count beyond any memory) leaves an engine without
+sensors, whose traces are refused, and costs the next call nothing: the same sensors set again are traced as by an engine
+that never failed."""
 import ctypes
 
 import numpy as np
@@ -42,3 +43,11 @@ def test_next_call_is_unharmed(refused, engine_lib, kgb):
             assert np.array_equal(e.download_bits(nc), o.download_bits(nc))
     finally:
         o.close()
+
+
+def test_nothing_to_trace(refused, engine_lib, kgb):
+    e, s, D = refused
+    for call in (lambda: e.trace(0, 1, engine_lib.ray_flags(False, False)), lambda: e.trace(0, len(s["P"]), engine_lib.ray_flags(False, True)),
+                 lambda: e.bounce(0, 1, 1, N=1, M=1, mf=1)):
+        with pytest.raises(kgb.KgbError, match="range exceeds the scene"):
+            call()
