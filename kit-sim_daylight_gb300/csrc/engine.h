@@ -131,9 +131,9 @@ int bounce_rest_blocks_per_sm();
 // with no room for the array). plain (with w64): every weight is zero or a positive normal float, so that the sums can
 // run in integer arithmetic (the same bits).
 inline bool plain_weights(const float* W, size_t n) {
-  bool ok = true;
-  for (size_t k = 0; k < n; ++k) ok &= W[k] == 0.f || (W[k] >= 1.17549435e-38f && W[k] <= 3.40282347e38f);
-  return ok;
+  for (size_t k = 0; k < n; ++k)
+    if (!(W[k] == 0.f || (W[k] >= 1.17549435e-38f && W[k] <= 3.40282347e38f))) return false;
+  return true;
 }
 void launch_reduce_bits(const uint32_t* bits, uint32_t nc, uint32_t nWords, uint32_t nDir, const float* N, const float* D, const float* W,
                         int useCos, double* out, cudaStream_t st, double* w64 = nullptr, bool plain = false);
