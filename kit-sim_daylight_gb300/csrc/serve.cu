@@ -73,10 +73,14 @@ __device__ __forceinline__ uint32_t find_seg(const Seg* segs, uint32_t nSegs, ui
   return lo;
 }
 
-// Tasks a warp takes at a time: the words of 32 sensors follow one another, so the second mostly finds the frontier made. The
-// daylight batches of a mixed stream of 32 requests, GPU time over nine passes with one / 2 / 4 / 8: 110 / 112 / 124 / 149 ms
-// (their tails); 119 ms in the form that made it for each task without the loop, which spilled 148 bytes against 20.
-constexpr uint32_t kBatchTasks = 2;
+// Tasks a warp takes at a time where a batch has more than kBatchMany for each warp of the grid: the words of 32 sensors
+// follow one another, so the second mostly finds the frontier made. The daylight batches of a mixed stream of 32 requests,
+// GPU time over nine passes with one / 2 / 4 / 8: 110 / 112 / 124 / 149 ms (their tails); 119 ms in the form that made it for
+// each task without the loop, which spilled 148 bytes against 20. Smaller batches go one by one: taken in pairs they
+// leave warps idle while others walk two tasks in turn. GPU time with pairs / one by one / with walks from the root: 4
+// requests of 5000 sensors x 14 directions 496 / 296 / 372 us, 32 of 500 x 200 1617 / 974 / 1224, 16 of 20,000 x 14
+// 712 / 556 / 710, 16 of 20,000 x 95 2617 / 2340 / 3136.
+constexpr uint32_t kBatchTasks = 2, kBatchMany = 4;
 // Three blocks an SM, as k_bits: left to itself the compiler gives this kernel 100 registers and two blocks an SM, and
 // the batch's trace ran 13 % longer than the single-request kernel on the same rays.
 __global__ void __launch_bounds__(256, 3) k_bits_batch(const BatchHdr* hdr, const Seg* segs, uint32_t* bitsPool, uint32_t* counter, uint32_t* status) {
@@ -86,14 +90,15 @@ __global__ void __launch_bounds__(256, 3) k_bits_batch(const BatchHdr* hdr, cons
   uint32_t overflow = 0, rays = 0;
   Count ctr;
   Frontier& f = frontier[threadIdx.x / 32];
+  const uint32_t take = nTasks > kBatchMany * 8 * gridDim.x ? kBatchTasks : 1u;
   for (;;) {
     uint32_t first = 0;
-    if (lane == 0) first = atomicAdd(counter, kBatchTasks);
+    if (lane == 0) first = atomicAdd(counter, take);
     first = __shfl_sync(~0u, first, 0);
     if (first >= nTasks) break;
     Bounds bounds{};
     uint32_t entries = 0, last = 0xffffffffu;   // the frontier's 32 sensors, by their first word's task
-    for (uint32_t task = first; task < min(first + kBatchTasks, nTasks); ++task) {
+    for (uint32_t task = first; task < min(first + take, nTasks); ++task) {
       const Seg& g = segs[find_seg(segs, nSegs, task, false)];
       const uint32_t local = task - g.taskBase, b = local / g.nWords, w = local % g.nWords, i = b * 32 + lane;
       const bool valid = i < g.n;
