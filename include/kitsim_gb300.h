@@ -400,8 +400,9 @@ KGB_API int kgb_set_builder(kgb_engine* e, int which);
  * them to their error returns. nodeLimit: the traversals of kgb_trace, kgb_view and kgb_bounce see only the BVH's first
  * nodeLimit nodes, and so at most nodeLimit + 8 node visits per query; a query that needs more gives up and the call
  * fails ("traversal gave up ...", the message of a walk past its visit cap; 0: every node, the cap then the node count
- * + 8, at most 2^20). bounceLimitNs: how long one bounce launch may run before it ends its remaining paths and
- * kgb_bounce fails ("... passed its ... limit ..."; 0: the default, 10 s; larger values are clamped to it).
+ * + 8, at most 2^20). bounceLimitNs: how long the kernel of a bounce launch's later segments
+ * may run before it ends its remaining paths; the launch is then made again with fewer of them, and kgb_bounce fails once
+ * few are too many ("... passed its ... limit ..."; 0: the default, 10 s; larger values are clamped to it).
  * seriesWaitNs: how long a wait of the tensor-core series pipeline (its producer, MMA issuer and epilogue on their
  * mbarriers) may last before the kernel records a timeout, finishes the copies and MMAs it issued, frees its TMEM and
  * ends, and kgb_series fails ("... timed out waiting ..."; 0: the default, 4 s; larger values are clamped to it).

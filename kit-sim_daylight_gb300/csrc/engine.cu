@@ -1251,11 +1251,14 @@ KGB_API int kgb_bounce(kgb_engine* e, size_t i0, size_t nc, uint32_t rayFlags, c
   a.dc = static_cast<float*>(g.dc.p); a.status = static_cast<uint32_t*>(g.ctl.p) + 1;
   a.limitNs = g.bounceLimitNs;
   // paths of a launch: at most 2^23 (their results 64 MiB, the queue of paths that go on 384 MiB)
-  const size_t nCap = std::max<size_t>(1, (size_t(1) << 23) / nc);
+  size_t nCap = std::max<size_t>(1, (size_t(1) << 23) / nc);
   if (!g.gridRest) g.gridRest = g.numSMs * bounce_rest_blocks_per_sm();
   // the reference starts at 2^13 / nc samples (1..64); here also at least ~16 paths per resident thread (a path a thread):
   // a few ms, in which a launch's last paths count little (20,011 sensors x 1024 paths: 3 launches, 10.6 ms; 5 from 4, 10.9)
   const size_t fill = (size_t(16) * size_t(g.numSMs) * 2048 + nc - 1) / nc;
+  // a launch past its time limit, which covers all later segments of its paths, is made again with a sixteenth of them, down
+  // to a sixteenth of what one launch per segment began with: a scene that kept each of those within the limit passes
+  const size_t least = std::max<size_t>(1, std::max(std::clamp<size_t>((size_t(1) << 13) / nc, 1, 64), fill / 4) / 16);
   for (size_t done = 0, n = std::max(std::clamp<size_t>((size_t(1) << 13) / nc, 1, 64), fill); done < b->M;) {
     if (b->cancel && b->cancel(b->cancelCtx)) return fail("cancelled");
     n = std::min({n, size_t(b->M) - done, nCap});
@@ -1279,6 +1282,11 @@ KGB_API int kgb_bounce(kgb_engine* e, size_t i0, size_t nc, uint32_t rayFlags, c
       where = "; first walk that gave up: sensor " + std::to_string(ctl[17]) + " sample " + std::to_string(ctl[18]) + " segment " +
               std::to_string(ctl[19]) + ", origin (" + f(20) + ", " + f(21) + ", " + f(22) + "), direction (" + f(23) + ", " + f(24) + ", " +
               f(25) + ")";
+    }
+    if ((ctl[1] & kStatusTimeout) && !(ctl[1] & ~kStatusTimeout) && n > least) {
+      nCap = std::max(least, n / 2);
+      n = std::max(least, n / 16);
+      continue;   // nothing was added to the rows
     }
     if (ctl[1] & kStatusTimeout) {
       char lim[32];

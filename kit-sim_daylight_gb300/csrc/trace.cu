@@ -563,10 +563,10 @@ __global__ void __launch_bounds__(128) k_bounce_rest(BounceArgs a) {
 // a sensor, 32 samples a round: the lane of a bin's first sample reads the bin's row, adds the round's contributions of
 // that bin in lane order and writes it. The rounds' reads are what it waits for; the next round's results are read ahead.
 // Against a thread a sensor with its results' reads grouped by eight: calls of 20,011 sensors x 1024 paths 10.7 to 10.4
-// ms, 5003 x 1024 3.00 to 2.67, 2000 x 1024 1.39 to 1.09, 30 x 4096 1.09 to 0.34.
+// ms, 5003 x 1024 3.00 to 2.67, 2000 x 1024 1.39 to 1.09, 30 x 4096 1.09 to 0.34. A launch past its time limit adds nothing.
 __global__ void __launch_bounds__(128) k_bounce_accum(BounceArgs a) {
   const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, S = a.s1 - a.s0;
-  if (i >= a.n) return;
+  if (i >= a.n || (*a.status & kStatusTimeout)) return;
   float* row = a.dc + i;
   const uint2 none = make_uint2(kNoBin, 0u);
   uint2 next = lane < S ? __ldg(a.contrib + size_t(lane) * a.n + i) : none;
@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(128) k_bounce_accum(BounceArgs a) {
 constexpr uint32_t kAccumFew = 16;
 __global__ void __launch_bounds__(64) k_bounce_accum_few(BounceArgs a) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
+  if (i >= a.n || (*a.status & kStatusTimeout)) return;
   constexpr uint32_t B = 8;
   float* row = a.dc + i;
   const uint32_t S = a.s1 - a.s0;
