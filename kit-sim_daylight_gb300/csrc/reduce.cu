@@ -553,18 +553,23 @@ static void launch_sum_warp(const S& t, uint32_t n, const float* W, double* w64,
   if (t.nc <= kBlockSensors && n >= kBlockDirs) k_sum_block<COS><<<t.nc, 32 * kBlockWords, 0, st>>>(t, n, parts, out);
   else k_sum_warp<COS><<<(t.nc + kSumWarps - 1) / kSumWarps, 32 * kSumWarps, 0, st>>>(t, n, parts, out);
 }
-// Which form is faster (152 SMs): the thread form waits some 70 ns a direction for its fma and its reads (bits without
-// the cosine; 110 ns with it, 140 and 180 ns bytes), whatever the sensors, until they fill the SMs; the warp form costs
-// a sensor 7 us / 100,000 for each word of 32 directions and for a hundred words' worth more at the start of its sum,
-// where nearly every term doubles it. Measured, both forms, us a call: 12,345 sensors x 5610 directions 793 / 378
-// (cosine), 485 / 329; 20,000 x 5610 753 / 556, 481 / 481; 40,000 x 5610 776 / 1016, 490 / 880; 12,345 x 2155
-// 289 / 194, 182 / 180; 12,000 x 100 45 / 67; bytes 20,011 x 9066 1772 / 842, 1382 / 712; 32,000 x 2155 477 / 477.
+// Which form is faster (152 SMs): the thread form waits so many ns a direction for its fma and its reads, whatever the
+// sensors, until they fill the SMs (bits of a city's facades, which see little of the sky, 42 and with the cosine 74, of a
+// block's 60 and 98; bytes 95 and 112, 119 and 157, a quarter more once they exceed the L2), and 6 us before; the warp form
+// costs a sensor 0.106 ns for each word of 32 directions and for fifty words' worth more at the start of its sum, where
+// nearly every term doubles it. The rates are about the mean of city's and block's ns over these 0.106 ns, so that near the line
+// neither scene loses more than it would gain. us a call, thread / warp, city and block: bits with the cosine 8000 x 1000
+// 91 / 88, 123 / 89; 12,345 x 2155 163 / 178, 234 / 174; 20,000 x 5033 362 / 457, 496 / 453; without 5000 x 1000 71 / 73,
+// 91 / 70; 8000 x 2155 110 / 125, 151 / 125; 12,345 x 5033 226 / 275, 309 / 269; bytes with the cosine 20,000 x 2155 263 / 264,
+// 328 / 269; 25,000 x 2155 249 / 316, 337 / 325; 29,000 x 9066 1254 / 1064, 1507 / 1050; without 16,000 x 2155 223 / 219,
+// 285 / 215; 20,000 x 2155 219 / 252, 266 / 254.
 // Under 256 directions the start of the sum is most of it (16 sensors x 15 directions: 5 us against 14).
-static bool warp_sums(uint32_t nc, uint32_t n, uint32_t rate) { return n >= 256 && uint64_t(nc) * (100 + n / 32) <= uint64_t(rate) * n; }
+static bool warp_sums(uint32_t nc, uint32_t n, uint64_t rate) { return n >= 256 && uint64_t(nc) * (50 + n / 32) <= rate * (n + 80); }
+constexpr uint64_t kL2Bytes = 96000000;   // from here on the L2 (129 MB) no longer holds them: 16,000 x 5033 119 ns a direction, 20,000 x 5033 135
 
 void launch_reduce_bits(const uint32_t* bits, uint32_t nc, uint32_t nWords, uint32_t nDir, const float* N, const float* D, const float* W,
                         int useCos, double* out, cudaStream_t st, double* w64, bool plain) {
-  if (w64 && plain && warp_sums(nc, nDir, useCos ? 1500 : 1000)) {
+  if (w64 && plain && warp_sums(nc, nDir, useCos ? 780 : 475)) {
     if (useCos) launch_sum_warp<true>(BitsTerms<true>{bits, nc, N, D}, nDir, W, w64, out, st);
     else launch_sum_warp<false>(BitsTerms<false>{bits, nc, N, D}, nDir, W, w64, out, st);
   } else if (w64) {
@@ -576,7 +581,7 @@ void launch_reduce_bits(const uint32_t* bits, uint32_t nc, uint32_t nWords, uint
 }
 void launch_reduce_bytes(const uint8_t* bytes, uint32_t nc, uint32_t nDir, const float* N, const float* D, const float* W, int useCos,
                          double* out, cudaStream_t st, double* w64, bool plain) {
-  if (w64 && plain && warp_sums(nc, nDir, useCos ? 2500 : 2000)) {
+  if (w64 && plain && warp_sums(nc, nDir, (useCos ? 1190 : 1000) * (uint64_t(nc) * nDir > kL2Bytes ? 5 : 4) / 4)) {
     if (useCos) launch_sum_warp<true>(BytesTerms<true>{bytes, nc, N, D}, nDir, W, w64, out, st);
     else launch_sum_warp<false>(BytesTerms<false>{bytes, nc, N, D}, nDir, W, w64, out, st);
   } else if (w64) {
