@@ -403,6 +403,7 @@ __global__ void __launch_bounds__(32 * kTreeletWarps) k_treelets(Tree2 T, int n,
       }
     }
     __threadfence();
+    __syncwarp();   // what a lane refit is read by all
     uint32_t todo = __ballot_sync(~0u, work);
     while (todo) {
       const int from = __ffs(todo) - 1;

@@ -1368,7 +1368,7 @@ KGB_API int kgb_view(kgb_engine* e, size_t i0, size_t nc, uint32_t rayFlags, con
   a.cls = static_cast<uint8_t*>(g.viewCls.p); a.dist = static_cast<float*>(g.viewDist.p);
   a.counter = static_cast<uint32_t*>(g.ctl.p); a.status = g.host;
   g.host[0] = 0;
-  // gpu.cu:590: sub-launches of at least 2^13 threads there; here at least four (32 sensors x word) tasks for each
+  // gpu.cu:590: sub-launches of at least 2^13 threads there; here at least four times 32 sensors x 32 cells for each
   // resident warp, so that no launch leaves the GPU idle; then ~40 ms, at most doubling, as the reference
   const size_t nMin = std::max<size_t>((size_t(1) << 13) / nWords, (size_t(4) * g.gridView * 8 * 32 + nWords - 1) / nWords);
   size_t n = std::max(*launch, nMin);

@@ -27,8 +27,7 @@ namespace kgb {
 //   (an empty slot holds lo = +inf, hi = -inf, which no ray enters)
 // The child boxes are plain floats: the box test reads a ray's near and far planes straight from the two vectors its
 // octant picks (Ray::nearX..: n1 or n3 for x; the far one is the index ^ 2), with no decoding. (The 80-byte form
-// with 8-bit child boxes of Ylitie, Karras and Laine 2017 spent most of the box test's instructions decoding bytes:
-// the test is 87 % of the any-hit walk's instructions.)
+// with 8-bit child boxes of Ylitie, Karras and Laine 2017 spent most of the box test's instructions decoding bytes.)
 // Triangle record, 48 bytes = 3 x 16 B: v0.xyz + primitive index | v1.xyz + flags | v2.xyz + slot.
 struct __align__(16) Node8 { uint4 n[kNodeWords / 4]; };
 static_assert(sizeof(Node8) == 4 * kNodeWords, "node record size");
@@ -729,7 +728,7 @@ __device__ __forceinline__ void frontier_hits(const Scene& s, const Frontier& fr
 // Bits of one visibility word, those of directions d0 .. dEnd - 1: bit d % 32 = direction d of a sensor (normal n, ray
 // origin o) passes the hemisphere cull and every hit from tmin 1e-5 on is an own-plane hit, at most 3 (the reference's
 // __raygen__bits, trace_dev.cu:91-108, restated over the ray's hit set). COUNT adds traversal counters and rays traced.
-// tab: the directions' precomputed RayDir entries, or null (the rays are made from D).
+// D: the directions, tab: their precomputed RayDir entries.
 template <bool COUNT>
 __device__ __forceinline__ uint32_t trace_word(const Scene& s, F3 n, F3 o, const float* D, const RayDir* tab, uint32_t d0, uint32_t dEnd,
                                                bool cull, uint32_t& overflow, Count& ctr, uint32_t& rays) {
@@ -737,7 +736,7 @@ __device__ __forceinline__ uint32_t trace_word(const Scene& s, F3 n, F3 o, const
   for (uint32_t d = d0; d < dEnd; ++d) {
     const F3 dir = ld3(D + 3 * d);
     if (!(n.x * dir.x + n.y * dir.y + n.z * dir.z > 0.f)) continue;
-    const Ray r = tab ? ray_from(tab, d, o) : make_ray(o, dir);
+    const Ray r = ray_from(tab, d, o);
     bool blocked = false;
     int own = 0;
     if (COUNT) ++rays;

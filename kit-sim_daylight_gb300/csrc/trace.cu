@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(128) k_bounce_paths(BounceArgs a) {
   uint32_t k = 0, diffuse = 0, bin = kNoBin, overflow = 0;
   bool reflected = false;
   const uint32_t at = (smp - a.s0) * a.n + i;
-  const bool go = bounce_segment(a, s, cull, 0, nn, gi, smp, o, d, w, k, diffuse, reflected, bin, gain, overflow) && a.nBounce + 16 > 1;
+  const bool go = bounce_segment(a, s, cull, 0, nn, gi, smp, o, d, w, k, diffuse, reflected, bin, gain, overflow);
   PathState st;
   if (go) {
     st.ox = o.x; st.oy = o.y; st.oz = o.z; st.gi = gi; st.dx = d.x; st.dy = d.y; st.dz = d.z; st.smp = smp;
