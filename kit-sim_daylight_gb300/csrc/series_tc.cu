@@ -184,6 +184,7 @@ struct TcSeg {
   uint32_t mBase, mTiles, nTiles;
   uint32_t tileBase;         // the launch's tiles tileBase .. tileBase + mTiles x nTiles - 1 are this contraction's
   uint32_t sunBase;          // k_series_sun's blocks sunBase .. sunBase + (row blocks x column blocks) - 1, likewise
+  uint32_t sunWarpRows;      // and the rows of a warp of these
 };
 constexpr uint32_t kMaxTcSegs = kMaxSeriesGroup;   // contractions of one launch: their tensor maps travel as kernel parameters
 struct TcGroup {
@@ -409,8 +410,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_series_tc(const __grid_constant_
 // sensors and turned through shared memory: the series kernels of 8200 sensors x 4456 steps 897 to 840 us (the call 1630
 // to 1595 us), of 29,609 with reflected light 5.26 to 5.09 ms, no difference for visibility as bytes. Beside the next
 // band's contraction, on a stream of its own, it got too few of an SM's registers to keep up and held back the downloads
-// (the 8200-sensor call 1710 us).
-constexpr uint32_t kSunRows = 64, kSunCols = 64, kSunWarpRows = 16;
+// (the 8200-sensor call 1710 us). Where even 4 rows a warp fill no more than half of the SMs' slots a warp takes 4, one round
+// of reads instead of four in turn: the kernels of 100 sensors x 24 steps 18.6 to 14.9 us, 23.2 to 17.0 with bytes.
+constexpr uint32_t kSunWarps = 4, kSunCols = 64, kSunWarpRows = 16, kSunFewRows = 4;   // a block's warps down its rows
 __device__ __forceinline__ uint32_t sun_seg_of(const TcGroup& g, uint32_t block) {
   uint32_t lo = 0, hi = g.nSegs - 1;
   while (lo < hi) {
@@ -423,9 +425,9 @@ __global__ void __launch_bounds__(256) k_series_sun(const __grid_constant__ TcGr
   const TcSeg& a = g.seg[sun_seg_of(g, blockIdx.x)];
   const uint32_t colBlocks = (a.T + kSunCols - 1) / kSunCols, local = blockIdx.x - a.sunBase;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t r0 = a.mBase * BM + (local / colBlocks) * kSunRows + (warp >> 1) * kSunWarpRows;
+  const uint32_t r0 = a.mBase * BM + ((local / colBlocks) * kSunWarps + (warp >> 1)) * a.sunWarpRows;
   const uint32_t t = (local % colBlocks) * kSunCols + (warp & 1) * 32 + lane;
-  const uint32_t rowEnd = min(min(a.nc, (a.mBase + a.mTiles) * BM), r0 + kSunWarpRows);
+  const uint32_t rowEnd = min(min(a.nc, (a.mBase + a.mTiles) * BM), r0 + a.sunWarpRows);
   const int j = t < a.T ? __ldg(a.sunOfCol + t) : -1;
   if (j < 0) return;
   const float sun[3] = {a.sunVec[3 * j], a.sunVec[3 * j + 1], a.sunVec[3 * j + 2]}, w = a.sunW[j];
@@ -588,7 +590,9 @@ static const char* tc_seg(const SeriesTcPlan& p, uint32_t mBase, uint32_t mCount
   a.mTiles = mCount; a.mBase = mBase; a.nTiles = (p.T + BN - 1) / BN; a.tileBase = tileBase;
   const uint32_t rows = std::min<uint32_t>(p.nc, (mBase + mCount) * BM) - mBase * BM;
   a.sunBase = sunBase;
-  sunBlocks = ((rows + kSunRows - 1) / kSunRows) * ((p.T + kSunCols - 1) / kSunCols);
+  const auto blocks = [&](uint32_t warpRows) { return ((rows + kSunWarps * warpRows - 1) / (kSunWarps * warpRows)) * ((p.T + kSunCols - 1) / kSunCols); };
+  a.sunWarpRows = blocks(kSunFewRows) <= 4 * uint32_t(p.numSMs) ? kSunFewRows : kSunWarpRows;
+  sunBlocks = blocks(a.sunWarpRows);
   a.sunOfCol = p.sunOfCol; a.sunVec = p.sunVec; a.sunW = p.sunW; a.sun0 = p.sun0;
   a.bits = p.bits; a.bytes = p.bytes; a.N = p.N; a.E = p.E;
   return nullptr;
