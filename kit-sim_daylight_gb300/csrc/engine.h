@@ -76,7 +76,7 @@ struct ViewArgs {
   uint32_t* status;
 };
 
-// k_bounce_rest ends its remaining paths, and the call fails, once it has run this long.
+// k_bounce_rest ends its remaining paths once it has run this long; its launch is made again with fewer (kgb_bounce).
 constexpr uint64_t kBounceLimitNs = 10000000000ull;   // 10 s
 
 struct PathState;   // a path between segments (trace.cu)
